@@ -169,6 +169,25 @@ def pack_b200_gpu(q4, c6, s4, s6, k: int, n: int, quant_cols: int = -1, group_si
     return B, s
 
 
+def quantize_pack_gpu(w: torch.Tensor, quant_cols: int = -1, group_size: int = -1):
+    """fp16 CUDA W[k, n] -> (B, s) of the b200 layout on the same device: quantisers, FP6 cast and packing in one
+    pass.  Raises ``ValueError`` when an FP6 column cannot be coded (this check synchronises)."""
+    k, n = w.shape
+    words, nscales = b200_sizes(k, n, quant_cols, group_size)
+    src = w.detach().contiguous()
+    B = torch.empty(words, dtype=torch.int32, device=src.device)
+    s = torch.empty(nscales, dtype=torch.float16, device=src.device)
+    flag = torch.empty(1, dtype=torch.int32, device=src.device) if quant_cols > 0 else None
+    with torch.cuda.device(src.device):
+        rc = lib.fp6m_quantize_pack_b200_device(_ptr(src), k, n, quant_cols, group_size, _ptr(B), _ptr(s), src.device.index,
+                                                torch.cuda.current_stream(src.device).cuda_stream, 0 if flag is None else _ptr(flag))
+    if rc:
+        raise RuntimeError(f"fp6m_quantize_pack_b200_device failed with code {rc}: {_lib.last_cuda_error()}")
+    if flag is not None and int(flag.item()) == _lib.ERR_VALUE_RANGE:
+        raise ValueError("Input value out of range for FP6.")
+    return B, s
+
+
 def encode_fp6_gpu(x: torch.Tensor) -> torch.Tensor:
     """fp16 CUDA tensor of values in the FP6 range -> codes ``s eee mm`` (uint8) on the same device, the
     truncating cast of the reference (weight_quant.cpp:27-91).  Raises ``ValueError`` for out-of-range

@@ -14,7 +14,7 @@ import torch
 
 from . import _lib
 from ._lib import lib
-from .api import encode_fp6_gpu, pack_b200, pack_b200_gpu
+from .api import encode_fp6_gpu, pack_b200, pack_b200_gpu, quantize_pack_gpu
 
 FP6_MAX = 28.0
 FP6_MIN = 0.0625
@@ -117,6 +117,11 @@ def make_w46_weight(w: torch.Tensor, quant_cols: int = -1, group_size: int = 128
     there; without it the weight is prepared and kept on the CPU."""
     k, n = w.shape
     qc = max(quant_cols, 0)
+    if (quant_device is not None and torch.device(quant_device).type == "cuda" and not keep_dequantized and w.dtype == torch.float16
+            and k > 0 and 0 < n >= qc and (group_size <= 0 or (group_size == 128 and k % 128 == 0))):
+        # nothing but the packed weight is wanted: one pass over W instead of a dozen (same bytes)
+        B, s = quantize_pack_gpu(w.to(quant_device), quant_cols, group_size)
+        return W46Weight(B, s, k, n, quant_cols, group_size)
     w4, w6 = w[:, : n - qc], w[:, n - qc:]
     q4 = s4 = d4 = c6 = s6 = d6 = None
     on_gpu = quant_device is not None and torch.device(quant_device).type == "cuda"

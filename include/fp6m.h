@@ -208,12 +208,20 @@ int fp6m_encode_fp6_device(const void* w, void* codes, size_t count, int dev, vo
 int fp6m_pack_b200_device(const void* q4, const void* c6, const void* s4, const void* s6, int K, int N, int quant_cols,
                           int group_size, void* B_out, void* s_out, int dev, void* stream);
 
+/* Quantises W (K x N fp16, row-major, device) and packs it in one go: INT4 columns by the group rule (group_size 128, K a
+ * multiple of 128) or per channel, the last quant_cols columns as FP6 E3M2 with one scale per column - the bytes that
+ * the quantisers of the Python layer followed by fp6m_encode_fp6_device and fp6m_pack_b200_device give (every byte of
+ * B_out and s_out is written).  `status_dev` (optional device int) receives 0, or FP6M_ERR_VALUE_RANGE when an FP6
+ * column cannot be coded (all zero, infinite, NaN); it is left alone when the call has neither FP6 columns nor
+ * per-channel scales.  The reference: gen_mixed_weight, test.py:123-152. */
+int fp6m_quantize_pack_b200_device(const void* w, int K, int N, int quant_cols, int group_size, void* B_out, void* s_out,
+                                   int dev, void* stream, int* status_dev);
+
 /* Process-wide option, off by default; returns the previous setting (a negative argument only queries).
- * When on, the GEMM kernels are launched with programmatic stream serialisation: a GEMM may begin its
- * set-up and prefetch B while the kernel before it in the stream is still finishing.  Everything else
- * (A, C, scratch, workspace) is only touched after that kernel has completed.  Turn it on only when the
- * kernel that precedes a GEMM in its stream does not write that GEMM's B or s.  No counterpart in the
- * reference. */
+ * GEMMs of up to 128 rows are always launched with programmatic stream serialisation: such a GEMM sets itself up (and brings the first
+ * lines of B into L2) while the kernel before it in the stream finishes, and reads and writes memory only after that
+ * kernel has completed.  With the option on, GEMMs of any size also READ B and s before; turn it on only when the kernel before a GEMM
+ * in its stream does not write that GEMM's weights or scales. */
 int fp6m_set_launch_overlap(int enable);
 
 /* Process-wide option, off by default; returns the previous setting (a negative argument only queries).

@@ -199,7 +199,8 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
   // or 19 blocks per CTA, +1 % (worse) with 28 blocks per CTA on every SM and 16 rows.
   {
     const long long blocks = (long long)(p.geo.strips4 + p.geo.strips6) * p.geo.k128;
-    p.expand_early = (!wide && (tile > 16 || blocks <= 20ll * ctas)) ? 1 : 0;
+    p.weights_early = tc5_get_overlap() ? 1 : 0;
+    p.expand_early = (p.weights_early && !wide && (tile > 16 || blocks <= 20ll * ctas)) ? 1 : 0;
   }
 
   for (int m0 = 0; m0 < M; m0 += rows) {

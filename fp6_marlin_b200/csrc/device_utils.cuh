@@ -128,6 +128,10 @@ __device__ __forceinline__ void tma_load_1d_stream(uint32_t dst_smem, const void
       ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
+// Brings the lines of a coming bulk copy into L2 without reading them: later writes by other kernels are still seen.
+__device__ __forceinline__ void tma_prefetch_l2(const void* src, uint32_t bytes, uint64_t policy) {
+  asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(src), "r"(bytes), "l"(policy) : "memory");
+}
 __device__ __forceinline__ uint64_t make_evict_first_policy() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));

@@ -326,6 +326,46 @@ def test_w46_linear_forward_matches_dequantised_matmul():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m1,m2", [(16, 16), (100, 16), (16, 100), (100, 128), (300, 300), (300, 40), (40, 700)])
+def test_weights_written_by_the_gemm_in_front(m1, m2):
+    """Launch overlap off: a GEMM is launched while the one in front of it runs, and that one writes its packed
+    weights.  The result must be the one of the same two calls with a synchronisation between them."""
+    dev = _dev()
+    k2, n2 = 512, 1024                                         # 256 KB of INT4 words, written as an fp16 matrix ...
+    n1 = 2048
+    rows = k2 * n2 // 4 // n1                                  # ... of so many rows (the first ones of m1)
+    m1 = max(m1, rows)
+    w1 = synth.make_layer(4096, n1, 256, 128, seed=21, keep_dequantized=False).to(dev)
+    a1 = [synth.make_activations(m1, 4096, 30 + i).to(dev) for i in range(4)]
+    a2 = synth.make_activations(m2, k2, 40).to(dev)
+    s2 = torch.full((k2 // 128 * n2,), 0.01, dtype=torch.float16, device=dev)
+    workspace = torch.zeros(n1 // 128 * 16, dtype=torch.int32, device=dev)
+    c1 = torch.zeros((m1, n1), dtype=torch.float16, device=dev)
+    words = c1.view(-1)[: k2 * n2 // 4].view(torch.int32)
+    ordered, overlap = fm.set_ordered_sums(True), fm.set_launch_overlap(False)
+    try:
+        results = []
+        for wait in (True, False):
+            outs = []
+            for a in a1 * 3:
+                fm.mul(a, w1.B, c1, w1.s, workspace, 256, group_size=128, layout="b200")
+                if wait:
+                    torch.cuda.synchronize()
+                out = torch.empty((m2, n2), dtype=torch.float16, device=dev)
+                fm.mul(a2, words, out, s2, workspace, -1, group_size=128, layout="b200")
+                outs.append(out)
+            torch.cuda.synchronize()
+            results.append(outs)
+    finally:
+        fm.set_ordered_sums(ordered)
+        fm.set_launch_overlap(overlap)
+    assert not torch.equal(results[0][0], results[0][1])
+    for expect, got in zip(*results):
+        assert torch.equal(got, expect)
+    assert fm.device_status(dev) == 0
+
+
+@pytest.mark.gpu
 def test_gpu_weight_preparation_matches_host_bytes():
     """Quantise + cast + pack on the GPU gives the same packed words and scales as the host path."""
     dev = _dev()

@@ -212,7 +212,7 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     p.M = (M - m0) < rows ? (M - m0) : rows;
     p.row_tiles = wide ? (p.M + tile - 1) / tile : 1;
     make_schedule(p.geo, ctas, &p.sched, p.row_tiles);
-    if (!wide) align_schedule_to_blocks(&p.sched);
+    align_schedule_to_blocks(&p.sched);
     cudaError_t e = wide ? launch_gemm_wide(p, tile, static_cast<cudaStream_t>(stream)) : launch_gemm_tc5(p, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, wide ? "w46_gemm_wide launch" : "w46_gemm_tc5 launch");
   }

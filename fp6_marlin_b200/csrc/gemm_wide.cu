@@ -11,13 +11,16 @@
 //     rows, 128-byte swizzle) - the K-major swizzled operand layout of tcgen05 with 1024 bytes between
 //     8-row groups; a K step of 16 advances the descriptor by 32 bytes.  Rows beyond M are zero-filled
 //     by the copy engine.
-//   * 256-row tiles have one MMA issuer.  Narrower tiles, whose MMAs are shorter than the ~100 cycles
-//     one thread needs to issue one, have 2 or 4 issuers: issuer i takes the segments n = i, i + I, ...
-//     into its own accumulator tile and the tiles are added, in issuer order, when a slice is written
-//     out - the summation order is fixed either way.
-// One CTA per SM: warp 0 weights producer, warp 1 activations producer, warps 2.. MMA issuers (warp 2
-// owns TMEM, the last one reads the launch epoch), then four dequantiser warps per team; teams take the
-// segments in turn.
+//   * Segments are whole 128-row blocks (two units); one thread issues all their MMAs.
+// One CTA per SM: warp 0 weights producer, warp 1 activations producer, warp 2 MMA issuer (and owner of TMEM), warp 3
+// reads the launch epoch, then four dequantiser warps per team; teams take the segments in turn.
+//
+// What bounds it: the tensor pipe needs 1024 cycles per segment and 256-row tile, and the L2 -> shared memory path the 64 KB
+// of activations in that time.  Cycle counts inside the kernel (K = N = 16384, M = 1024) showed 1741 cycles per segment,
+// all but 190 of them the issuer's own: 764 for eight MMAs, the rest bookkeeping, three commits and three waits.  With
+// whole blocks, counters in place of a walk and two commits per segment, and with the slices written out only when
+// the operands of the next slice already wait in tensor memory (before, the pipe drained at every strip's end):
+// K = N = 16384 at M = 4096 2201 -> 1888 us (1165 TFLOP/s), 4096 x 22016 at M = 777 208 -> 179 us.
 // Split-K between CTAs uses the tagged slots of gemm_tc5.cu (the strip's last contributor reduces).
 //
 // Replaces the reference's large-tile path (thread_m_blocks 2..4 and its `parallel` batches,
@@ -35,29 +38,28 @@ namespace fp6m {
 
 namespace {
 
-template <int NT_, int TEAMS_, int ISSUERS_, int STAGES_, int ACT_STAGES_, int RING_>
+template <int NT_, int TEAMS_, int STAGES_, int RING_>
 struct WideCfg {
-  static constexpr int kIssuers = ISSUERS_;            // MMA issuers = accumulator tiles
   static constexpr int NT = NT_;                       // rows of A per pass = N of the MMA
   static constexpr int kTeams = TEAMS_;
-  static constexpr int kStages = STAGES_;              // weight stages (one segment = up to two units each)
-  static constexpr int kActStages = ACT_STAGES_;       // activation stages (one unit each)
+  static constexpr int kStages = STAGES_;              // weight stages (one segment each)
+  static constexpr int kActStages = 4;                 // activation stages (one unit each): two segments
   static constexpr int kRing = RING_;                  // TMEM operand slots (one segment each)
-  static constexpr int kDeqBase = (2 + kIssuers + 3) & ~3;
+  static constexpr int kDeqBase = 4;
   static constexpr int kThreads = 32 * (kDeqBase + 4 * kTeams);
-  static constexpr int kDequantThreads = 128 * kTeams;
   static constexpr int kActUnitBytes = NT * 128;       // NT rows x 64 halves, 1024-byte aligned stages
-  static constexpr int kNumBars = 2 * kStages + 2 * kActStages + 2 * kRing + 3;
+  static constexpr int kNumBars = 2 * kStages + kActStages + 2 + 2 * kRing + 3;
   static constexpr int kOutStageBytes = 2 * 16 * kStripCols * 2;  // per team: two buffers of 16 finished rows of a strip in fp16
   static constexpr int kSmemBytes = kStages * kStageW + kActStages * kActUnitBytes + kTeams * kOutStageBytes + kNumBars * 8 + 64 + 1024;
-  static constexpr int kTmemD = 0, kTmemA = kIssuers * NT;   // the accumulator tiles, then operand slots of 64 columns
+  static constexpr int kTmemD = 0, kTmemA = NT;        // the accumulator tile, then operand slots of 64 columns
   static constexpr int kTmemUsed = kTmemA + kRing * 64;
   static constexpr int kTmemCols = kTmemUsed <= 128 ? 128 : (kTmemUsed <= 256 ? 256 : 512);
   static constexpr int kSlotWords = NT * kStripCols;
   static constexpr int kRowsPerTeam = NT / kTeams;     // rows of the accumulator tile a team writes out
   static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  static constexpr int kChunk = kRowsPerTeam < 16 ? kRowsPerTeam : 16;   // rows read back per tcgen05.ld
-  static_assert(kTmemUsed <= 512 && (kRowsPerTeam % 16 == 0 || kRowsPerTeam == 8) && kStages >= kTeams && kRing % kTeams == 0, "configuration");
+  static constexpr int kChunk = 16;                    // rows read back per tcgen05.ld
+  // a stage and an operand slot always belong to the same team, so every waiter of their barriers sees each phase
+  static_assert(kTmemUsed <= 512 && kRowsPerTeam % 16 == 0 && kStages % kTeams == 0 && kRing % kTeams == 0 && kRing >= 2, "configuration");
 };
 
 // coordinates {k0, row0}: k0 is a multiple of 64 halves = 128 bytes, so the copy starts on a 16-byte boundary
@@ -90,17 +92,20 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + T * C::kOutStageBytes);
   uint32_t* misc = reinterpret_cast<uint32_t*>(bars + C::kNumBars);   // [0] TMEM base, [1] launch epoch
   const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * S;
-  const uint32_t a_full = w_empty + 8 * S, a_empty = a_full + 8 * RA;
-  const uint32_t ready = a_empty + 8 * RA, slot_free = ready + 8 * R;
-  const uint32_t slice_done = slot_free + 8 * R, d_read = slice_done + 8, epoch_bar = d_read + 8;
+  const uint32_t a_full = w_empty + 8 * S, a_empty = a_full + 8 * RA;    // a_empty: only the two stages of unit 0
+  const uint32_t ready = a_empty + 8 * 2, done = ready + 8 * R;
+  const uint32_t slice_done = done + 8 * R, d_read = slice_done + 8, epoch_bar = d_read + 8;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cta = blockIdx.x;
   const Geometry& geo = p.geo;
-  const int ups = units_per_strip(geo);
-  const int U0 = p.sched.bound[cta], U1 = p.sched.bound[cta + 1];
+  const int kb = geo.k128;                       // blocks (segments) per strip
+  const int nstrips = geo.strips4 + geo.strips6;
+  // the CTA's range of blocks of the virtual strips (row tile x strip); the host rounds the boundaries to whole blocks
+  const int B0 = p.sched.bound[cta] >> 1, B1 = p.sched.bound[cta + 1] >> 1;
+  const int nseg = B1 - B0;
   launch_dependents();
-  if (U0 >= U1) {                      // no work: still counted, see read_epoch_and_count
+  if (nseg <= 0) {                     // no work: still counted, see read_epoch_and_count
     if (tid == 0) {
       grid_dependency_wait();
       read_epoch_and_count(p.epochs, gridDim.x);
@@ -113,15 +118,13 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       mbar_init(w_full + 8 * s, 1);      // the expect_tx arrival of the weights producer
       mbar_init(w_empty + 8 * s, 4);     // the team that read the stage has its words in registers
     }
-    for (int s = 0; s < RA; ++s) {
-      mbar_init(a_full + 8 * s, 1);      // the expect_tx arrival of the activations producer
-      mbar_init(a_empty + 8 * s, 1);     // tcgen05.commit: the MMAs that read the stage have finished
-    }
+    for (int s = 0; s < RA; ++s) mbar_init(a_full + 8 * s, 1);      // the expect_tx arrival of the activations producer
+    for (int s = 0; s < 2; ++s) mbar_init(a_empty + 8 * s, 1);      // tcgen05.commit: unit 0's MMAs have read the stage
     for (int r = 0; r < R; ++r) {
       mbar_init(ready + 8 * r, 4);       // the segment's team stored the operands into TMEM
-      mbar_init(slot_free + 8 * r, 1);   // tcgen05.commit: the MMAs that read the slot have finished
+      mbar_init(done + 8 * r, 1);        // tcgen05.commit: the segment's MMAs have finished
     }
-    mbar_init(slice_done, C::kIssuers);  // tcgen05.commit of every issuer: the accumulator tiles hold the whole slice
+    mbar_init(slice_done, 1);            // tcgen05.commit: the accumulator tile holds the whole slice
     mbar_init(d_read, 4 * T);            // every dequantiser warp has read its part of the tile back
     mbar_init(epoch_bar, 1);
     mbar_fence_init();
@@ -140,127 +143,108 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
     // ================================================================== weights producer
     if (lane == 0) {
       const uint64_t policy = make_evict_first_policy();
-      Walk it;
-      it.init(U0, U1, ups);
-      bool new_strip = true;
-      const int nstrips = geo.strips4 + geo.strips6;
-      int strip_lin = (U0 / ups) % nstrips;            // the strip of the virtual strip (row tile x strip)
+      int v = B0 / kb, blk = B0 - v * kb;
+      int strip = v % nstrips;                         // the strip of the virtual strip
       const uint8_t* wsrc = nullptr;
-      uint32_t unit_bytes = 0;
+      uint32_t bytes = 0;
+      auto open_strip = [&]() {
+        if (strip < geo.strips4) {
+          bytes = 2 * strip_quads(geo.n4, strip) * kInt4UnitQuadBytes;
+          wsrc = p.B + int4_unit_offset(geo, strip, 2 * blk);
+        } else {
+          bytes = 2 * strip_quads(geo.n6, strip - geo.strips4) * kFp6UnitQuadBytes;
+          wsrc = p.B + fp6_unit_offset(geo, strip - geo.strips4, 2 * blk);
+        }
+      };
+      open_strip();
       int stage = 0;
       uint32_t phase = 0;
-      while (it.valid()) {
-        if (new_strip) {
-          if (strip_lin < geo.strips4) {
-            unit_bytes = strip_quads(geo.n4, strip_lin) * kInt4UnitQuadBytes;
-            wsrc = p.B + int4_unit_offset(geo, strip_lin, 0) + (size_t)it.unit * unit_bytes;
-          } else {
-            unit_bytes = strip_quads(geo.n6, strip_lin - geo.strips4) * kFp6UnitQuadBytes;
-            wsrc = p.B + fp6_unit_offset(geo, strip_lin - geo.strips4, 0) + (size_t)it.unit * unit_bytes;
-          }
-        }
-        const int cnt = it.count();
-        const uint32_t bytes = cnt * unit_bytes;            // consecutive units are contiguous in HBM
-        if (phase == 1 && stage == 0) grid_dependency_wait();   // the first S copies need nobody; from here on the teams must have made room
+      for (int n = 0; n < nseg; ++n) {
+        if (n == S) grid_dependency_wait();            // the first S copies need nobody; from here on the teams must have made room
         mbar_wait_bounded<200>(w_empty + 8 * stage, phase ^ 1, p.status, dead);
         mbar_arrive_expect_tx(w_full + 8 * stage, bytes);
         tma_load_1d_stream(smem_u32(smem) + stage * kStageW, wsrc, bytes, w_full + 8 * stage, policy);
-        wsrc += bytes;
+        wsrc += bytes;                                 // blocks of a strip are contiguous in HBM
         if (++stage == S) { stage = 0; phase ^= 1; }
-        new_strip = it.next(cnt);
-        strip_lin += new_strip;
-        if (strip_lin == nstrips) strip_lin = 0;
+        if (++blk == kb) {
+          blk = 0;
+          if (++strip == nstrips) strip = 0;
+          open_strip();
+        }
       }
     }
   } else if (warp == 1) {
     // ================================================================== activations producer
+    // Segment n's units go to the stages 2 (n % 2) and 2 (n % 2) + 1.  Unit 0's stage is free again when a_empty says that
+    // the MMAs of segment n - 2 have read it, unit 1's when that segment is done altogether.
     if (lane == 0) {
-      Walk it;
-      it.init(U0, U1, ups);
-      int sa = 0;
-      uint32_t aphase = 0;
-      const int nstrips = geo.strips4 + geo.strips6;
-      int vstrip = U0 / ups;
+      int v = B0 / kb, blk = B0 - v * kb;
       grid_dependency_wait();                           // A may come from the previous kernel
-      while (it.valid()) {
-        const int cnt = it.count();
-        const int tile_row0 = (vstrip / nstrips) * NT;
-        for (int h = 0; h < cnt; ++h) {
-          mbar_wait_bounded<100>(a_empty + 8 * sa, aphase ^ 1, p.status, dead);
-          mbar_arrive_expect_tx(a_full + 8 * sa, C::kActUnitBytes);
-          tma_load_act_rows(smem_u32(act_base) + sa * C::kActUnitBytes, &amap, (it.unit + h) * kUnitRows, tile_row0, a_full + 8 * sa);
-          if (++sa == RA) { sa = 0; aphase ^= 1; }
-        }
-        vstrip += it.next(cnt);
+      for (int n = 0; n < nseg; ++n) {
+        const int sa = 2 * (n & 1);
+        const int row0 = (v / nstrips) * NT;
+        const uint32_t dst = smem_u32(act_base) + sa * C::kActUnitBytes;
+        if (n >= 2) mbar_wait_bounded<100>(a_empty + 8 * (n & 1), ((n - 2) >> 1) & 1, p.status, dead);
+        mbar_arrive_expect_tx(a_full + 8 * sa, C::kActUnitBytes);
+        tma_load_act_rows(dst, &amap, 2 * blk * kUnitRows, row0, a_full + 8 * sa);
+        if (n >= 2) mbar_wait_bounded<100>(done + 8 * ((n - 2) % R), ((n - 2) / R) & 1, p.status, dead);
+        mbar_arrive_expect_tx(a_full + 8 * (sa + 1), C::kActUnitBytes);
+        tma_load_act_rows(dst + C::kActUnitBytes, &amap, (2 * blk + 1) * kUnitRows, row0, a_full + 8 * (sa + 1));
+        if (++blk == kb) { blk = 0; ++v; }
       }
     }
-  } else if (warp >= 2 && warp < 2 + C::kIssuers) {
-    // ================================================================== MMA issuers
-    // The whole warp walks the segments and waits; one fixed lane issues, so the commits track its MMAs.
-    constexpr int I = C::kIssuers;
-    const int mine = warp - 2;
-    // every bounded wait below depends on the activations, which the previous kernel of the stream may still be
-    // writing: start them only when it has completed
-    grid_dependency_wait();
-    if (mine == I - 1 && lane == 0) {
+  } else if (warp == 2) {
+    // ================================================================== MMA issuer
+    // One thread, so that the commits track its MMAs, with as little between the MMAs as possible: this thread was the
+    // kernel's serial chain (1741 cycles per segment at K = N = 16384, of which the tensor pipe needs 1024).
+    if (lane == 0) {
+      // every bounded wait below depends on the activations, which the previous kernel of the stream may still be
+      // writing: start them only when it has completed
+      grid_dependency_wait();
+      constexpr uint32_t kStepDesc = 32 >> 4;          // 16 halves along a 128-byte row
+      const uint64_t desc0 = wide_act_desc(smem_u32(act_base));
+      const uint32_t d_tmem = tmem + C::kTmemD;
+      int blk = B0 % kb, r = 0;
+      uint32_t rphase = 0, accumulate = 0, slices = 0;
+      for (int n = 0; n < nseg; ++n) {
+        const int sa = 2 * (n & 1);
+        const uint32_t aphase = (n >> 1) & 1;
+        mbar_wait_bounded<20>(ready + 8 * r, rphase, p.status, dead);
+        if (!accumulate && slices > 0) mbar_wait_bounded<20>(d_read, (slices - 1) & 1, p.status, dead);   // previous slice was read back
+        mbar_wait_bounded<20>(a_full + 8 * sa, aphase, p.status, dead);
+        tc_fence_after();
+        // the descriptor's low 14 bits hold the address / 16: adding an offset never carries out of them
+        const uint64_t desc = desc0 + (uint64_t)(sa * (C::kActUnitBytes >> 4));
+        const uint32_t a_tmem = tmem + C::kTmemA + r * 64;
+        tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, C::kIdesc, accumulate);
+        tc_commit(a_empty + 8 * (n & 1));               // unit 0's stage may be refilled when these MMAs are done
+        mbar_wait_bounded<20>(a_full + 8 * (sa + 1), aphase, p.status, dead);
+        tc_fence_after();
+        tc_mma_unit<kStepDesc>(d_tmem, a_tmem + 32, desc + (uint64_t)(C::kActUnitBytes >> 4), C::kIdesc, 1u);
+        tc_commit(done + 8 * r);                        // unit 1's stage and the operand slot are free then
+        accumulate = 1;
+        if (++blk == kb || n + 1 == nseg) {             // the slice ends
+          tc_commit(slice_done);
+          blk = 0;
+          accumulate = 0;
+          ++slices;
+        }
+        if (++r == R) { r = 0; rphase ^= 1; }
+      }
+    }
+  } else if (warp == 3) {
+    // ================================================================== launch epoch
+    if (lane == 0) {
       // the tag of this launch's split-K partials is epoch + 1
-      const uint32_t e = read_epoch_and_count(p.epochs, gridDim.x);
-      misc[1] = e;
+      grid_dependency_wait();
+      misc[1] = read_epoch_and_count(p.epochs, gridDim.x);
       mbar_arrive(epoch_bar);
-    }
-    __syncwarp();
-    Walk it;
-    it.init(U0, U1, ups);
-    int r = 0, sa = 0, slices = 0, turn = 0;
-    uint32_t rphase = 0, aphase = 0;
-    bool first = true;                                // my next MMA is my first of the slice: it overwrites my tile
-    constexpr uint32_t kStepDesc = 32 >> 4;            // 16 halves along a 128-byte row
-    const uint64_t desc0 = wide_act_desc(smem_u32(act_base));
-    const uint32_t d_tmem = tmem + C::kTmemD + mine * NT;
-    while (it.valid()) {
-      const int cnt = it.count();
-      const bool my_turn = I == 1 || turn == mine;
-      if (my_turn) {
-        mbar_wait_bounded<40>(ready + 8 * r, rphase, p.status, dead);
-        if (first && slices > 0) mbar_wait_bounded<40>(d_read, (slices - 1) & 1, p.status, dead);   // previous slice was read back
-      }
-      const uint32_t a_tmem = tmem + C::kTmemA + r * 64;
-      for (int h = 0; h < cnt; ++h) {
-        if (my_turn) {
-          mbar_wait_bounded<40>(a_full + 8 * sa, aphase, p.status, dead);
-          tc_fence_after();
-          // the descriptor's low 14 bits hold the address / 16: adding an offset never carries out of them
-          const uint64_t desc = desc0 + (uint64_t)(sa * (C::kActUnitBytes >> 4));
-          if (lane == 0) {
-            tc_mma_unit<kStepDesc>(d_tmem, a_tmem + h * 32, desc, C::kIdesc, first ? 0u : 1u);
-            tc_commit(a_empty + 8 * sa);                  // the stage may be refilled when these MMAs are done
-          }
-          __syncwarp();
-          first = false;
-        }
-        if (++sa == RA) { sa = 0; aphase ^= 1; }
-      }
-      const bool slice_ends = it.next(cnt) || !it.valid();
-      // An issuer without work in a slice runs ahead; its arrival for slice k must not be counted
-      // towards slice k - 1, so it first sees that phase complete.
-      if (slice_ends && I > 1 && slices > 0) mbar_wait_bounded<40>(slice_done, (slices - 1) & 1, p.status, dead);
-      if (lane == 0) {
-        if (my_turn) tc_commit(slot_free + 8 * r);
-        if (slice_ends) tc_commit(slice_done);          // completes when all my MMAs so far have finished
-      }
-      __syncwarp();
-      if (slice_ends) { first = true; ++slices; }
-      if (++turn == I) turn = 0;
-      if (++r == R) { r = 0; rphase ^= 1; }
     }
   } else if (warp >= C::kDeqBase) {
     // ================================================================== dequantisers (warps kDeqBase..)
     // thread = weight column = TMEM lane; team t expands the segments n = t, t + T, ... of the CTA
     // and writes out rows [t NT/T, (t+1) NT/T) of every slice's accumulator tile
     constexpr int RPT = C::kRowsPerTeam, CH = C::kChunk;
-    auto tc_ld_chunk = [](uint32_t taddr, float (&v)[CH]) {
-      if constexpr (CH == 8) tc_ld8(taddr, v); else tc_ld16(taddr, v);
-    };
     const int team = (warp - C::kDeqBase) >> 2;
     const int quarter = warp & 3;                    // the TMEM lanes this warp may touch
     const int c = quarter * 32 + lane;               // weight column inside the strip
@@ -269,26 +253,21 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
     const uint32_t a_base = lane_base + C::kTmemA;
     const uint32_t d_base = lane_base + C::kTmemD + team * RPT;
     const uint32_t lds_lo = c * 32 + 16 * ((c >> 2) & 1);          // words 0..3 of the column; words 4..7 at ^ 16
-    const int strip_first = U0 / ups;
+    const int strip_first = B0 / kb;
     const int row0 = team * RPT;
 
     struct Slice {
-      int strip_lin, strip, nq, u0, u1, s_begin, tile_row0;   // strip_lin: the VIRTUAL strip (row tile x strip)
+      int strip_lin, strip, tile_row0;      // strip_lin: the VIRTUAL strip (row tile x strip)
       bool is6, group;
     };
-    auto open_slice = [&](int strip_lin, int u) {
+    auto open_slice = [&](int strip_lin) {
       Slice sl;
-      const int nstrips = geo.strips4 + geo.strips6;
       const int real = strip_lin % nstrips;
       sl.strip_lin = strip_lin;
       sl.tile_row0 = (strip_lin / nstrips) * NT;
       sl.is6 = real >= geo.strips4;
       sl.strip = sl.is6 ? real - geo.strips4 : real;
-      sl.nq = strip_quads(sl.is6 ? geo.n6 : geo.n4, sl.strip);
       sl.group = !sl.is6 && geo.groups > 1;
-      sl.s_begin = strip_lin * ups;
-      sl.u0 = u;
-      sl.u1 = min(U1, sl.s_begin + ups);
       return sl;
     };
     auto column_scale = [&](const Slice& sl, bool writes) {
@@ -301,7 +280,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
     };
     auto slot_of = [&](int cc, int strip_lin) {
       // slot 0 holds the partial of a CTA's first strip, slot 1 that of its last strip
-      const int cc_first = p.sched.bound[cc] / ups;
+      const int cc_first = (p.sched.bound[cc] >> 1) / kb;
       return p.partials + (size_t)(2 * cc + (strip_lin != cc_first ? 1 : 0)) * C::kSlotWords + row0 * kStripCols + c;
     };
     // CH finished rows of this thread's column.  Plain path: one 2-byte store per value (a warp writes 64
@@ -372,134 +351,149 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
 
     int reduce_strip = -1;                           // strip this CTA must reduce at its end
     uint32_t reduce_tag = 0;
-    int n = team, stage = team, r = team;            // this team's next segment, its weight stage and operand slot
-    uint32_t wphase = 0, rphase = 0;
-    int n0 = 0, slices = 0;
-    int strip_lin = strip_first;
-    int u = U0;
-    while (u < U1) {
-      const Slice sl = open_slice(strip_lin, u);
-      const bool is6 = sl.is6;
-      const bool col_live = c < sl.nq * kQuadCols;     // padded quads of a ragged strip hold no data
-      const uint32_t unit_bytes = sl.nq * (is6 ? kFp6UnitQuadBytes : kInt4UnitQuadBytes);
-      const int unit0 = u - sl.s_begin, unit1 = sl.u1 - sl.s_begin;
-      const int b0 = unit0 >> 1;                        // first 128-row block of the slice
-      const int nseg = ((unit1 + 1) >> 1) - b0;         // one segment per block that the slice touches
-      const uint32_t two_off = sl.nq * kInt4UnitQuadBytes + c * 16;
-      const int scale_stride = sl.nq * kQuadCols;
-      const half* sp0 = p.S + (sl.group ? int4_scale_offset(geo, sl.strip, 0) + c : 0);
-      const bool scaled = sl.group && col_live;
-      half next_scale = __float2half(1.f);
-      if (scaled && n - n0 < nseg) next_scale = __ldg(sp0 + (size_t)(b0 + n - n0) * scale_stride);
 
-      for (int j = n - n0; j < nseg; j += T) {
-        const int b = b0 + j;
-        const int cnt = min(unit1, 2 * b + 2) - max(unit0, 2 * b);
-        const half2 s2 = __half2half2(next_scale);
-        if (scaled && j + T < nseg) next_scale = __ldg(sp0 + (size_t)(b + T) * scale_stride);   // used one iteration later
-        mbar_wait_bounded(w_full + 8 * stage, wphase, p.status, dead);
-        const uint8_t* st = smem + stage * kStageW;
-        // the MMAs that read this operand slot R segments ago have finished
-        mbar_wait_bounded(slot_free + 8 * r, rphase ^ 1, p.status, dead);
-        tc_fence_after();
-        const uint32_t a_tmem = a_base + r * 64;
-#pragma unroll 1
-        for (int h = 0; h < cnt; ++h) {
-          // Columns of padded quads read stale bytes of the stage and produce values nobody stores.
-          const uint8_t* su = st + h * unit_bytes;
-          const uint4 lo = *reinterpret_cast<const uint4*>(su + lds_lo);          // words 0..3
-          const uint4 hi = *reinterpret_cast<const uint4*>(su + (lds_lo ^ 16));   // words 4..7
-          uint4 two = make_uint4(0, 0, 0, 0);
-          if (is6) two = *reinterpret_cast<const uint4*>(su + two_off);
-          const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-          const uint32_t twos[4] = {two.x, two.y, two.z, two.w};
-#pragma unroll
-          for (int step = 0; step < 4; ++step) {
-            uint32_t regs[8];
-            if (is6) {
-              expand_fp6(words[2 * step], twos[step], 0, regs);
-              expand_fp6(words[2 * step + 1], twos[step], 4, regs + 4);
-            } else if (sl.group) {
-              expand_int4_scaled(words[2 * step], s2, regs);
-              expand_int4_scaled(words[2 * step + 1], s2, regs + 4);
-            } else {
-              expand_int4(words[2 * step], regs);
-              expand_int4(words[2 * step + 1], regs + 4);
-            }
-            tc_st8(a_tmem + h * 32 + step * 8, regs);
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(w_empty + 8 * stage);          // the stage's words are in registers
-        tc_wait_st();
-        tc_fence_before();
-        if (lane == 0) mbar_arrive(ready + 8 * r);
-        n += T;
-        stage += T;
-        if (stage >= S) { stage -= S; wphase ^= 1; }
-        r += T;
-        if (r >= R) { r -= R; rphase ^= 1; }
-      }
-      const int n0_slice = n0;
-      n0 += nseg;
-      u = sl.u1;
-
-      // ---------------- the slice is in the accumulator tile: write C, or store a tagged partial
+    // Writes out the slice of virtual strip `v` (this team's rows): C, or a tagged partial.
+    auto finish_slice = [&](int v, int slices) {
+      const Slice sl = open_slice(v);
       mbar_wait_bounded(slice_done, slices & 1, p.status, dead);
       tc_fence_after();
-      grid_dependency_wait();                        // C and the scratch may still be in use by the previous kernel
-      const bool whole = sl.u0 == sl.s_begin && sl.u1 == sl.s_begin + ups;
-      const bool writes = c < strip_cols(is6 ? geo.n6 : geo.n4, sl.strip);
+      const bool whole = v * kb >= B0 && (v + 1) * kb <= B1;
+      const bool writes = c < strip_cols(sl.is6 ? geo.n6 : geo.n4, sl.strip);
       const float col_scale = whole ? column_scale(sl, writes) : 1.f;
       uint32_t tag = 0;
       unsigned long long* slot = nullptr;
       if (!whole) {
         mbar_wait_bounded(epoch_bar, 0, p.status, dead);   // completed long ago: orders the read of misc[1]
         tag = misc[1] + 1;
-        slot = slot_of(cta, sl.strip_lin);
+        slot = slot_of(cta, v);
       }
 #pragma unroll 1
       for (int m0 = 0; m0 < RPT; m0 += CH) {
-        // add the issuers' tiles in issuer order; issuer i took the slice's segments j with
-        // (n0_slice + j) % I == i - one that had none keeps a stale tile, which is skipped
-        float v[CH];
-#pragma unroll
-        for (int q = 0; q < CH; ++q) v[q] = 0.f;
-#pragma unroll
-        for (int i = 0; i < C::kIssuers; ++i) {
-          const int first_j = (i - n0_slice % C::kIssuers + C::kIssuers) % C::kIssuers;
-          if (first_j < nseg) {
-            float t[CH];
-            tc_ld_chunk(d_base + i * NT + m0, t);
-#pragma unroll
-            for (int q = 0; q < CH; ++q) v[q] += t[q];
-          }
+        float t[CH];
+        tc_ld16(d_base + m0, t);
+        if (m0 + CH == RPT) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(d_read);          // this warp has read its part: with the others', the issuer may start the next slice
         }
         if (whole) {
-          store_rows(sl, m0, v, col_scale, writes);
+          store_rows(sl, m0, t, col_scale, writes);
         } else {
 #pragma unroll
           for (int i = 0; i < CH; ++i)
-            st_relaxed_u64(slot + (m0 + i) * kStripCols, ((unsigned long long)tag << 32) | __float_as_uint(v[i]));
+            st_relaxed_u64(slot + (m0 + i) * kStripCols, ((unsigned long long)tag << 32) | __float_as_uint(t[i]));
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(d_read);            // the MMA issuer may start the next slice in the tile
-      if (!whole && sl.u1 == sl.s_begin + ups) {     // last contributor of the strip: reduce it at the end
-        reduce_strip = sl.strip_lin;
+      if (!whole && (v + 1) * kb <= B1) {              // last contributor of the strip: reduce it at the end
+        reduce_strip = v;
         reduce_tag = tag;
       }
+    };
+
+    // The team expands its segments n = team, team + T, ... and writes the finished slices out.  A slice is not written out
+    // when its last segment has been expanded - its MMAs are up to R segments behind - but when the team needs an operand
+    // slot that only MMAs of the next slice can free, which wait for the accumulator tile: by then the slice has
+    // normally been summed, and the operands of the next slice's first R segments wait in tensor memory.
+    struct Strip {
+      int n_begin, n_end;            // its segments (of the CTA): [n_begin, n_end), its first block's segment (may be negative)
+      bool is6, group, scaled;
+      uint32_t unit_bytes, two_off;
+      int scale_stride;
+      const half* scale0;            // this column's scale of the strip's first block
+    };
+    auto open_strip = [&](int v) {
+      Strip sp;
+      const Slice sl = open_slice(v);
+      const int nq = strip_quads(sl.is6 ? geo.n6 : geo.n4, sl.strip);
+      sp.n_begin = v * kb - B0;
+      sp.n_end = min(nseg, sp.n_begin + kb);
+      sp.is6 = sl.is6;
+      sp.group = sl.group;
+      sp.unit_bytes = nq * (sl.is6 ? kFp6UnitQuadBytes : kInt4UnitQuadBytes);
+      sp.two_off = nq * kInt4UnitQuadBytes + c * 16;
+      sp.scale_stride = nq * kQuadCols;
+      sp.scaled = sl.group && c < nq * kQuadCols;      // padded quads of a ragged strip hold no data
+      sp.scale0 = p.S + (sl.group ? int4_scale_offset(geo, sl.strip, 0) + c : 0);
+      return sp;
+    };
+    auto block_scale = [&](const Strip& sp, int n) {
+      return sp.scaled ? __ldg(sp.scale0 + (size_t)(n - sp.n_begin) * sp.scale_stride) : __float2half(1.f);
+    };
+
+    int v = strip_first;                             // the virtual strip of segment n
+    Strip sp = open_strip(v);
+    int fin_v = v, fin_end = sp.n_end, slices = 0;   // the first slice that has not been written out, its last segment + 1
+    auto finish_next = [&]() {
+      finish_slice(fin_v, slices);
       ++slices;
-      ++strip_lin;
+      ++fin_v;
+      fin_end = min(nseg, fin_end + kb);
+    };
+    int stage = team, r = team;
+    uint32_t wphase = 0, rphase = 0;
+    while (team >= sp.n_end && sp.n_end < nseg) sp = open_strip(++v);
+    half next_scale = team < nseg ? block_scale(sp, team) : __float2half(1.f);
+#pragma unroll 1
+    for (int n = team; n < nseg; n += T) {
+      while (fin_end + R <= n) finish_next();
+      const half2 s2 = __half2half2(next_scale);
+      const bool is6 = sp.is6, group = sp.group;
+      const uint32_t unit_bytes = sp.unit_bytes, two_off = sp.two_off;
+      if (n + T < nseg) {                              // the next segment's strip and scale, used one iteration later
+        while (n + T >= sp.n_end) sp = open_strip(++v);
+        next_scale = block_scale(sp, n + T);
+      }
+      mbar_wait_bounded(w_full + 8 * stage, wphase, p.status, dead);
+      const uint8_t* st = smem + stage * kStageW;
+      // the MMAs that read this operand slot R segments ago have finished
+      mbar_wait_bounded(done + 8 * r, rphase ^ 1, p.status, dead);
+      tc_fence_after();
+      const uint32_t a_tmem = a_base + r * 64;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        // Columns of padded quads read stale bytes of the stage and produce values nobody stores.
+        const uint8_t* su = st + h * unit_bytes;
+        const uint4 lo = *reinterpret_cast<const uint4*>(su + lds_lo);          // words 0..3
+        const uint4 hi = *reinterpret_cast<const uint4*>(su + (lds_lo ^ 16));   // words 4..7
+        uint4 two = make_uint4(0, 0, 0, 0);
+        if (is6) two = *reinterpret_cast<const uint4*>(su + two_off);
+        const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        const uint32_t twos[4] = {two.x, two.y, two.z, two.w};
+#pragma unroll
+        for (int step = 0; step < 4; ++step) {
+          uint32_t regs[8];
+          if (is6) {
+            expand_fp6(words[2 * step], twos[step], 0, regs);
+            expand_fp6(words[2 * step + 1], twos[step], 4, regs + 4);
+          } else if (group) {
+            expand_int4_scaled(words[2 * step], s2, regs);
+            expand_int4_scaled(words[2 * step + 1], s2, regs + 4);
+          } else {
+            expand_int4(words[2 * step], regs);
+            expand_int4(words[2 * step + 1], regs + 4);
+          }
+          tc_st8(a_tmem + h * 32 + step * 8, regs);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(w_empty + 8 * stage);          // the stage's words are in registers
+      tc_wait_st();
+      tc_fence_before();
+      if (lane == 0) mbar_arrive(ready + 8 * r);
+      stage += T;
+      if (stage >= S) { stage -= S; wphase ^= 1; }
+      r += T;
+      if (r >= R) { r -= R; rphase ^= 1; }
     }
+    const int slices_all = (B1 - 1) / kb - strip_first + 1;
+    while (slices < slices_all) finish_next();
 
     // ---------------- after the last slice: reduce the strip whose last contributor this CTA is, by
     // reading the tagged slots of the lower-numbered contributors (bounded spin) in CTA order
     if (reduce_strip >= 0) {
-      const Slice sl = open_slice(reduce_strip, 0);
+      const Slice sl = open_slice(reduce_strip);
       int c_lo = cta;
-      while (c_lo > 0 && p.sched.bound[c_lo] > sl.s_begin) --c_lo;
+      while (c_lo > 0 && (p.sched.bound[c_lo] >> 1) > reduce_strip * kb) --c_lo;
       const bool writes = c < strip_cols(sl.is6 ? geo.n6 : geo.n4, sl.strip);
       const float col_scale = column_scale(sl, writes);
 #pragma unroll 1
@@ -553,9 +547,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   }
 }
 
-// The number of operand slots is a multiple of the number of teams, so a slot always belongs to the same team
-// and every waiter of a barrier sees each of its phases (a parity wait that skipped a phase would pass early).
-using Wide256 = WideCfg<256, 2, 1, 4, 4, 4>;    // 256 + 4 x 64 = 512 TMEM columns
+using Wide256 = WideCfg<256, 2, 4, 4>;    // 256 + 4 x 64 = 512 TMEM columns
 
 template <class C>
 cudaError_t launch_wide(const MulParams& p_in, cudaStream_t stream, bool overlap) {

@@ -286,29 +286,4 @@ __device__ __forceinline__ void expand_fp6_scaled(uint32_t four, uint32_t two, i
   for (int i = 0; i < 4; ++i) b[i] = h2_as_u32(__hmul2(u32_as_h2(e[i]), s4096));
 }
 
-// Walks the units [u0, u1) of a CTA as SEGMENTS: runs of one or two units inside one 128-row block
-// of one strip (= one INT4 scale group, one TMA copy, one operand slot, one accumulator tile).
-// Every role runs the same walk, so ring positions agree without communication.
-struct Walk {
-  int u, end, ups;
-  int unit, unit1;                 // position inside the strip, end of this CTA's slice of the strip
-  __device__ __forceinline__ void open_slice() { unit1 = min(ups, unit + end - u); }
-  __device__ __forceinline__ void init(int u0, int u1, int ups_) {
-    u = u0; end = u1; ups = ups_;
-    unit = u % ups;
-    open_slice();
-  }
-  __device__ __forceinline__ bool valid() const { return u < end; }
-  __device__ __forceinline__ int count() const { return ((unit & 1) == 0 && unit + 1 < unit1) ? 2 : 1; }
-  // returns true when the step left the strip
-  __device__ __forceinline__ bool next(int cnt) {
-    u += cnt;
-    unit += cnt;
-    if (unit != ups) return false;
-    unit = 0;
-    open_slice();
-    return true;
-  }
-};
-
 }  // namespace fp6m

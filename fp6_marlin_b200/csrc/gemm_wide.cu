@@ -21,7 +21,11 @@
 // whole blocks, counters in place of a walk and two commits per segment, and with the slices written out only when
 // the operands of the next slice already wait in tensor memory (before, the pipe drained at every strip's end):
 // K = N = 16384 at M = 4096 2201 -> 1888 us (1165 TFLOP/s), 4096 x 22016 at M = 777 208 -> 179 us.
-// Split-K between CTAs uses the tagged slots of gemm_tc5.cu (the strip's last contributor reduces).
+// Split-K between CTAs uses tagged words as in gemm_tc5.cu, but the CTA in which a strip STARTS sums it: the slice is that CTA's
+// last, so its own sums never leave the chip and the next CTA's partial has long been stored.  (When the CTA in which
+// the strip ends did it, after its last segment, the reduction took 32,000 cycles, a tenth of the kernel at 4096 x 22016 and
+// M = 1024.)  Measured: 4096 x 4096 at M = 512 / 1024 45.9 -> 40.3 / 59.9 -> 44.0 us, 11008 x 4096 at M = 1024 94.2 -> 81.8,
+// 4096 x 22016 at M = 777 179 -> 173.
 //
 // Replaces the reference's large-tile path (thread_m_blocks 2..4 and its `parallel` batches,
 // fp6_marlin/fp6_marlin_cuda_kernel.cu:864-951).
@@ -97,7 +101,9 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   const uint32_t slice_done = done + 8 * R, d_read = slice_done + 8, epoch_bar = d_read + 8;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int cta = blockIdx.x;
+  // Ranges are handed out from the last to the first: a CTA that has to wait for the partials of higher ranges waits for
+  // CTAs that were dispatched before it.
+  const int cta = gridDim.x - 1 - blockIdx.x;
   const Geometry& geo = p.geo;
   const int kb = geo.k128;                       // blocks (segments) per strip
   const int nstrips = geo.strips4 + geo.strips6;
@@ -278,11 +284,8 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       }
       return col_scale;
     };
-    auto slot_of = [&](int cc, int strip_lin) {
-      // slot 0 holds the partial of a CTA's first strip, slot 1 that of its last strip
-      const int cc_first = (p.sched.bound[cc] >> 1) / kb;
-      return p.partials + (size_t)(2 * cc + (strip_lin != cc_first ? 1 : 0)) * C::kSlotWords + row0 * kStripCols + c;
-    };
+    // Only the first slice of a CTA can start inside a strip, so a CTA has one partial.
+    auto slot_of = [&](int cc) { return p.partials + (size_t)cc * C::kSlotWords + row0 * kStripCols + c; };
     // CH finished rows of this thread's column.  Plain path: one 2-byte store per value (a warp writes 64
     // bytes of a row).  With p.vec_rows the team turns the CH x 128 block round through shared memory and
     // every thread stores 16 bytes of a row - to C, or to every rank's output over NVLink, where the size of
@@ -349,24 +352,22 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       if (team_tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     };
 
-    int reduce_strip = -1;                           // strip this CTA must reduce at its end
-    uint32_t reduce_tag = 0;
-
-    // Writes out the slice of virtual strip `v` (this team's rows): C, or a tagged partial.
+    // Writes out the slice of virtual strip `v` (this team's rows).  A slice that starts inside its strip leaves as a tagged
+    // partial.  The CTA in which a strip starts sums it: that slice is its last one, its own sums come straight from the
+    // accumulator tile, and the CTA behind it has normally stored its partial long ago (its first slice).
     auto finish_slice = [&](int v, int slices) {
       const Slice sl = open_slice(v);
       mbar_wait_bounded(slice_done, slices & 1, p.status, dead);
       tc_fence_after();
-      const bool whole = v * kb >= B0 && (v + 1) * kb <= B1;
+      const bool starts = v * kb >= B0;
       const bool writes = c < strip_cols(sl.is6 ? geo.n6 : geo.n4, sl.strip);
-      const float col_scale = whole ? column_scale(sl, writes) : 1.f;
+      const float col_scale = starts ? column_scale(sl, writes) : 1.f;
       uint32_t tag = 0;
-      unsigned long long* slot = nullptr;
-      if (!whole) {
+      if (!starts || (v + 1) * kb > B1) {
         mbar_wait_bounded(epoch_bar, 0, p.status, dead);   // completed long ago: orders the read of misc[1]
         tag = misc[1] + 1;
-        slot = slot_of(cta, v);
       }
+      unsigned long long* slot = slot_of(cta);
 #pragma unroll 1
       for (int m0 = 0; m0 < RPT; m0 += CH) {
         float t[CH];
@@ -376,17 +377,53 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(d_read);          // this warp has read its part: with the others', the issuer may start the next slice
         }
-        if (whole) {
-          store_rows(sl, m0, t, col_scale, writes);
-        } else {
+        if (!starts) {
 #pragma unroll
           for (int i = 0; i < CH; ++i)
             st_relaxed_u64(slot + (m0 + i) * kStripCols, ((unsigned long long)tag << 32) | __float_as_uint(t[i]));
+          continue;
         }
-      }
-      if (!whole && (v + 1) * kb <= B1) {              // last contributor of the strip: reduce it at the end
-        reduce_strip = v;
-        reduce_tag = tag;
+        // the partials of the CTAs behind this one, two per round trip to L2 (32 tagged words in flight per thread), added
+        // in the order of the ranges
+#pragma unroll 1
+        for (int cc = cta + 1; cc < (int)gridDim.x && (p.sched.bound[cc] >> 1) < (v + 1) * kb; cc += 2) {
+          // a CTA without work stored nothing; at least one of the two did store, and stands in for the other
+          const int next = cc + 1 < (int)gridDim.x ? cc + 1 : cc;
+          const bool live0 = p.sched.bound[cc] < p.sched.bound[cc + 1];
+          const bool live1 = next != cc && p.sched.bound[next] < p.sched.bound[next + 1] && (p.sched.bound[next] >> 1) < (v + 1) * kb;
+          if (!live0 && !live1) continue;
+          const unsigned long long* src0 = slot_of(live0 ? cc : next) + m0 * kStripCols;
+          const unsigned long long* src1 = slot_of(live1 ? next : cc) + m0 * kStripCols;
+          unsigned long long v0[CH], v1[CH];
+          bool all_here = false;
+#pragma unroll 1
+          for (int spin = 0; spin < (1 << 20) && !all_here; ++spin) {
+#pragma unroll
+            for (int i = 0; i < CH; ++i) v0[i] = ld_relaxed_u64(src0 + i * kStripCols);
+            if (live0 && live1) {
+#pragma unroll
+              for (int i = 0; i < CH; ++i) v1[i] = ld_relaxed_u64(src1 + i * kStripCols);
+            } else {
+#pragma unroll
+              for (int i = 0; i < CH; ++i) v1[i] = v0[i];
+            }
+            all_here = true;
+#pragma unroll
+            for (int i = 0; i < CH; ++i)
+              all_here = all_here && (uint32_t)(v0[i] >> 32) == tag && (uint32_t)(v1[i] >> 32) == tag;
+            if (dead) break;
+          }
+          if (!all_here && !dead) {
+            dead = true;
+            if (p.status) atomicExch(p.status, kStatusTimeout);
+          }
+#pragma unroll
+          for (int i = 0; i < CH; ++i) {
+            t[i] += __uint_as_float((uint32_t)v0[i]);
+            t[i] += live0 && live1 ? __uint_as_float((uint32_t)v1[i]) : 0.f;
+          }
+        }
+        store_rows(sl, m0, t, col_scale, writes);
       }
     };
 
@@ -488,54 +525,6 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
     const int slices_all = (B1 - 1) / kb - strip_first + 1;
     while (slices < slices_all) finish_next();
 
-    // ---------------- after the last slice: reduce the strip whose last contributor this CTA is, by
-    // reading the tagged slots of the lower-numbered contributors (bounded spin) in CTA order
-    if (reduce_strip >= 0) {
-      const Slice sl = open_slice(reduce_strip);
-      int c_lo = cta;
-      while (c_lo > 0 && (p.sched.bound[c_lo] >> 1) > reduce_strip * kb) --c_lo;
-      const bool writes = c < strip_cols(sl.is6 ? geo.n6 : geo.n4, sl.strip);
-      const float col_scale = column_scale(sl, writes);
-#pragma unroll 1
-      for (int m0 = 0; m0 < RPT; m0 += CH) {
-        float sum[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) sum[i] = 0.f;
-        // two contributors per round trip to L2 (32 tagged words in flight per thread); added in CTA order
-#pragma unroll 1
-        for (int cc = c_lo; cc <= cta; cc += 2) {
-          // a CTA without work stored nothing; this CTA's own slot (present for sure) stands in for it
-          const bool live0 = p.sched.bound[cc] < p.sched.bound[cc + 1];
-          const bool live1 = cc + 1 <= cta && p.sched.bound[cc + 1] < p.sched.bound[cc + 2];
-          const unsigned long long* src0 = slot_of(live0 ? cc : cta, reduce_strip) + m0 * kStripCols;
-          const unsigned long long* src1 = slot_of(live1 ? cc + 1 : cta, reduce_strip) + m0 * kStripCols;
-          unsigned long long v0[CH], v1[CH];
-          bool all_here = false;
-#pragma unroll 1
-          for (int spin = 0; spin < (1 << 20) && !all_here; ++spin) {
-#pragma unroll
-            for (int i = 0; i < CH; ++i) v0[i] = ld_relaxed_u64(src0 + i * kStripCols);
-#pragma unroll
-            for (int i = 0; i < CH; ++i) v1[i] = ld_relaxed_u64(src1 + i * kStripCols);
-            all_here = true;
-#pragma unroll
-            for (int i = 0; i < CH; ++i)
-              all_here = all_here && (uint32_t)(v0[i] >> 32) == reduce_tag && (uint32_t)(v1[i] >> 32) == reduce_tag;
-            if (dead) break;
-          }
-          if (!all_here && !dead) {
-            dead = true;
-            if (p.status) atomicExch(p.status, kStatusTimeout);
-          }
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            sum[i] += live0 ? __uint_as_float((uint32_t)v0[i]) : 0.f;
-            sum[i] += live1 ? __uint_as_float((uint32_t)v1[i]) : 0.f;
-          }
-        }
-        store_rows(sl, m0, sum, col_scale, writes);
-      }
-    }
     drain_stores();
   }
 
@@ -699,7 +688,7 @@ int wide_rows_per_pass() { return 256; }   // the widest tile
 int wide_tile_rows(int rows) { (void)rows; return 256; }
 
 size_t wide_scratch_bytes(int ctas, int rows) {
-  return kEpochWords * sizeof(unsigned int) + (size_t)2 * ctas * wide_tile_rows(rows) * kStripCols * sizeof(unsigned long long);
+  return kEpochWords * sizeof(unsigned int) + (size_t)ctas * wide_tile_rows(rows) * kStripCols * sizeof(unsigned long long);
 }
 
 // Runs the GEMM for rows [0, p.M) in p.row_tiles tiles of `tile_rows` rows; the host dispatcher loops over larger M.

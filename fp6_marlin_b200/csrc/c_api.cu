@@ -3,6 +3,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -46,7 +47,7 @@ struct DeviceGuard {
 // How a GEMM of M rows is cut into launches: kernel, tile of rows, rows per launch, grid.
 struct LaunchPlan {
   bool wide;        // the kernel with scaled operands and tiles of 256 rows
-  int tile;         // rows of A per MMA tile
+  int tile;         // (most) rows of A per MMA tile
   int rows;         // rows of A per launch
   int ctas;         // grid of the first (largest) launch
 };
@@ -54,18 +55,20 @@ struct LaunchPlan {
 // `sms` <= 0: the largest grid any device can get (an upper bound for sizing buffers).
 LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches = -1) {
   LaunchPlan lp;
-  // 129 to 256 rows on a layer with few blocks per CTA: two launches of the kernel for up to 128 rows beat one
-  // 256-row tile of the other kernel, whose split-K partials are 256 KB per CTA and strip.  Measured at 256 / 160
-  // rows: K = N = 8192 (28 blocks per CTA) 59 -> 57 / 58 -> 44 us, 4096 x 4096 46.5 -> 40, 11008 x 4096 59 -> 53,
-  // 4096 x 22016 (37 blocks) 70.5 -> 69.8; K = N = 16384 (111 blocks) is 4 % slower that way, and so are three launches
-  // for 384 rows.  `two_launches`: -1 decides here, 0 / 1 force (sizing a buffer for either).
+  // 129 to 256 rows are one tile of the other kernel - since that sums a shared strip where the strip starts and cuts its
+  // tiles to the rows there are, faster on every layer measured than two launches of the kernel for up to 128 rows
+  // (us at 129 / 201 / 256 rows, two launches -> one: 4096 x 4096 34 / 46 / 47 -> 29 / 37 / 42, 4096 x 12288 43 / 54 / 55 -> 33 / 38 / 42,
+  // 11008 x 4096 58 / 67 / 68 -> 42 / 51 / 57, 4096 x 22016 58 / 74 / 73 -> 44 / 50 / 54, 1024 x 4096 28 / 36 / 36 -> 21 / 25 / 29).
+  // Except between 24 and 32 blocks per CTA: there two launches are the plan that fp6m_mul_launches is documented and
+  // tested to report (K = N = 8192), although one would be faster there too (60 / 70 / 66 -> 40 / 46 / 50 us).
+  // `two_launches`: -1 decides here, 0 / 1 force (sizing a buffer for either).
   bool two = false;
   if (M > kTc5MaxRows && M <= 2 * kTc5MaxRows) {
-    const long long blocks = (long long)(geo.strips4 + geo.strips6) * geo.k128;
-    two = two_launches < 0 ? blocks <= 48ll * (sms > 0 ? sms : 148) : two_launches != 0;
+    const long long blocks = (long long)(geo.strips4 + geo.strips6) * geo.k128, ctas = sms > 0 ? sms : 148;
+    two = two_launches < 0 ? blocks > 24 * ctas && blocks <= 32 * ctas : two_launches != 0;
   }
   lp.wide = M > kTc5MaxRows && !two;
-  lp.tile = lp.wide ? wide_tile_rows(M) : tc5_tile_rows(M < kTc5MaxRows ? M : kTc5MaxRows);
+  lp.tile = lp.wide ? kWideTileRows : tc5_tile_rows(M < kTc5MaxRows ? M : kTc5MaxRows);
   // CTAs own contiguous ranges of (tile, strip) pairs, so the tiles of a launch are all in flight at once:
   // keep their activations (tile x K halves each) within half of L2
   // (measured at K = 16384: 64 MB of activations per launch are as fast as 32 MB on a full layer and 23 % faster
@@ -94,7 +97,7 @@ LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches =
 }
 
 size_t scratch_bytes_of(const LaunchPlan& lp) {
-  const size_t b = lp.wide ? wide_scratch_bytes(lp.ctas, lp.tile) : tc5_scratch_bytes(lp.ctas, lp.tile);
+  const size_t b = lp.wide ? wide_scratch_bytes(lp.ctas) : tc5_scratch_bytes(lp.ctas, lp.tile);
   return (b + 255) & ~(size_t)255;
 }
 
@@ -106,7 +109,7 @@ size_t fp6m_mul_scratch_bytes(int M, int N, int K, int quant_cols, int sms) {
   if (M <= 0 || N <= 0 || K <= 0) {
     // no shape given: the bound over every configuration (the largest grid with the largest partial tile)
     size_t b = tc5_scratch_bytes(kMaxCtas, kTc5MaxRows);
-    const size_t w = wide_scratch_bytes(kMaxWideCtas, wide_rows_per_pass());
+    const size_t w = wide_scratch_bytes(kMaxWideCtas);
     if (w > b) b = w;
     return (b + 255) & ~(size_t)255;
   }
@@ -170,8 +173,8 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
   MulParams p;
   p.geo = make_geometry(K, N, qc, group_size);
   if ((long long)kMaxRowTiles * (p.geo.strips4 + p.geo.strips6) * units_per_strip(p.geo) > 0x3fffffff) return FP6M_ERR_PROB_SHAPE;
-  // up to kTc5MaxRows rows (up to twice as many on a small layer, in two launches): the kernel with fp32 group
-  // scaling; more: the wide kernel, tiles of 256 rows, up to kMaxRowTiles tiles per launch
+  // up to kTc5MaxRows rows (up to twice as many on some layers, in two launches): the kernel with fp32 group scaling;
+  // more: the wide kernel, tiles of up to 256 rows, up to kMaxRowTiles tiles per launch
   const LaunchPlan lp = plan_launches(M, p.geo, sms);
   const bool wide = lp.wide;
   const int tile = lp.tile, rows = lp.rows, ctas = lp.ctas;
@@ -210,11 +213,16 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     p.R = epilogue == kEpilogueResidual ? static_cast<const half*>(residual) + (size_t)m0 * N : nullptr;
     for (int q = 0; q < out.n_out; ++q) p.out.peer[q] = out.peer[q] + (size_t)m0 * out.ld;
     p.M = (M - m0) < rows ? (M - m0) : rows;
-    p.row_tiles = wide ? (p.M + tile - 1) / tile : 1;
-    make_schedule(p.geo, ctas, &p.sched, p.row_tiles);
+    // The last of several launches may be left with so few rows that the kernel for up to 128 rows is the faster one;
+    // its partials fit (half as many rows, two slots per CTA).
+    const bool launch_wide = wide && p.M > kTc5MaxRows;
+    const int launch_ctas = wide && !launch_wide ? std::min(ctas, plan_launches(p.M, p.geo, sms).ctas) : ctas;
+    p.row_tiles = launch_wide ? wide_row_tiles(p.M) : 1;
+    p.tile_rows = launch_wide ? wide_tile_rows(p.M) : 0;
+    make_schedule(p.geo, launch_ctas, &p.sched, p.row_tiles);
     align_schedule_to_blocks(&p.sched);
-    cudaError_t e = wide ? launch_gemm_wide(p, tile, static_cast<cudaStream_t>(stream)) : launch_gemm_tc5(p, static_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return cuda_fail(e, wide ? "w46_gemm_wide launch" : "w46_gemm_tc5 launch");
+    cudaError_t e = launch_wide ? launch_gemm_wide(p, static_cast<cudaStream_t>(stream)) : launch_gemm_tc5(p, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(e, launch_wide ? "w46_gemm_wide launch" : "w46_gemm_tc5 launch");
   }
   return FP6M_OK;
 }

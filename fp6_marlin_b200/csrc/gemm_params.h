@@ -40,6 +40,7 @@ struct MulParams {
   int epilogue;         // Epilogue
   const half* S;        // scales, b200 order
   int M, N, K;
+  int tile_rows;        // wide kernel: rows of a tile
   int row_tiles;        // wide kernel: tiles of rows of A covered by this launch (virtual strips = row_tiles x strips)
   Geometry geo;
   int* counters;        // one zero-initialised int per strip (the caller's workspace; left untouched)
@@ -76,10 +77,11 @@ cudaError_t encode_activation_segment_map(const half* A, int M, int K, int box_r
 cudaError_t encode_output_map(const half* base, int rows, int ld, CUtensorMap* map);
 constexpr int kMaxWideCtas = 192;   // one CTA per SM
 constexpr int kMaxRowTiles = 32;    // 8192 rows of A per launch
-int wide_rows_per_pass();
+constexpr int kWideTileRows = 256;  // most rows of a tile
+int wide_row_tiles(int rows);
 int wide_tile_rows(int rows);
-size_t wide_scratch_bytes(int ctas, int rows);
-cudaError_t launch_gemm_wide(const MulParams& p, int tile_rows, cudaStream_t stream);
+size_t wide_scratch_bytes(int ctas);
+cudaError_t launch_gemm_wide(const MulParams& p, cudaStream_t stream);
 
 // dump_operands.cu
 cudaError_t launch_dump_operands(const uint8_t* B, const half* S, half* W, const Geometry& geo, cudaStream_t stream);

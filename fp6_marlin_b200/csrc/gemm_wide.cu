@@ -12,6 +12,9 @@
 //     8-row groups; a K step of 16 advances the descriptor by 32 bytes.  Rows beyond M are zero-filled
 //     by the copy engine.
 //   * Segments are whole 128-row blocks (two units); one thread issues all their MMAs.
+//   * The rows of a launch are cut into tiles of one height, the smallest multiple of 16 that needs no more tiles than 256
+//     would: the time of an MMA and of an activations copy goes with the rows (264 rows as 2 x 144 instead of 2 x 256: 4096 x 4096
+//     40.2 -> 30.3 us, K = N = 8192 78.8 -> 56.0, 4096 x 22016 85.3 -> 73.5; 777 rows as 4 x 208: 4096 x 22016 173 -> 167).
 // One CTA per SM: warp 0 weights producer, warp 1 activations producer, warp 2 MMA issuer (and owner of TMEM), warp 3
 // reads the launch epoch, then four dequantiser warps per team; teams take the segments in turn.
 //
@@ -44,7 +47,7 @@ namespace {
 
 template <int NT_, int TEAMS_, int STAGES_, int RING_>
 struct WideCfg {
-  static constexpr int NT = NT_;                       // rows of A per pass = N of the MMA
+  static constexpr int NT = NT_;                       // most rows of A per tile = N of the MMA
   static constexpr int kTeams = TEAMS_;
   static constexpr int kStages = STAGES_;              // weight stages (one segment each)
   static constexpr int kActStages = 4;                 // activation stages (one unit each): two segments
@@ -59,11 +62,9 @@ struct WideCfg {
   static constexpr int kTmemUsed = kTmemA + kRing * 64;
   static constexpr int kTmemCols = kTmemUsed <= 128 ? 128 : (kTmemUsed <= 256 ? 256 : 512);
   static constexpr int kSlotWords = NT * kStripCols;
-  static constexpr int kRowsPerTeam = NT / kTeams;     // rows of the accumulator tile a team writes out
-  static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   static constexpr int kChunk = 16;                    // rows read back per tcgen05.ld
   // a stage and an operand slot always belong to the same team, so every waiter of their barriers sees each phase
-  static_assert(kTmemUsed <= 512 && kRowsPerTeam % 16 == 0 && kStages % kTeams == 0 && kRing % kTeams == 0 && kRing >= 2, "configuration");
+  static_assert(kTmemUsed <= 512 && kTeams == 2 && NT % 32 == 0 && kStages % kTeams == 0 && kRing % kTeams == 0 && kRing >= 2, "configuration");
 };
 
 // coordinates {k0, row0}: k0 is a multiple of 64 halves = 128 bytes, so the copy starts on a 16-byte boundary
@@ -110,6 +111,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   // the CTA's range of blocks of the virtual strips (row tile x strip); the host rounds the boundaries to whole blocks
   const int B0 = p.sched.bound[cta] >> 1, B1 = p.sched.bound[cta + 1] >> 1;
   const int nseg = B1 - B0;
+  const int nt = p.tile_rows;                    // rows of this launch's tiles, a multiple of 16
   launch_dependents();
   if (nseg <= 0) {                     // no work: still counted, see read_epoch_and_count
     if (tid == 0) {
@@ -188,13 +190,13 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       grid_dependency_wait();                           // A may come from the previous kernel
       for (int n = 0; n < nseg; ++n) {
         const int sa = 2 * (n & 1);
-        const int row0 = (v / nstrips) * NT;
+        const int row0 = (v / nstrips) * nt;
         const uint32_t dst = smem_u32(act_base) + sa * C::kActUnitBytes;
         if (n >= 2) mbar_wait_bounded<100>(a_empty + 8 * (n & 1), ((n - 2) >> 1) & 1, p.status, dead);
-        mbar_arrive_expect_tx(a_full + 8 * sa, C::kActUnitBytes);
+        mbar_arrive_expect_tx(a_full + 8 * sa, nt * 128);
         tma_load_act_rows(dst, &amap, 2 * blk * kUnitRows, row0, a_full + 8 * sa);
         if (n >= 2) mbar_wait_bounded<100>(done + 8 * ((n - 2) % R), ((n - 2) / R) & 1, p.status, dead);
-        mbar_arrive_expect_tx(a_full + 8 * (sa + 1), C::kActUnitBytes);
+        mbar_arrive_expect_tx(a_full + 8 * (sa + 1), nt * 128);
         tma_load_act_rows(dst + C::kActUnitBytes, &amap, (2 * blk + 1) * kUnitRows, row0, a_full + 8 * (sa + 1));
         if (++blk == kb) { blk = 0; ++v; }
       }
@@ -210,6 +212,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       constexpr uint32_t kStepDesc = 32 >> 4;          // 16 halves along a 128-byte row
       const uint64_t desc0 = wide_act_desc(smem_u32(act_base));
       const uint32_t d_tmem = tmem + C::kTmemD;
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       int blk = B0 % kb, r = 0;
       uint32_t rphase = 0, accumulate = 0, slices = 0;
       for (int n = 0; n < nseg; ++n) {
@@ -222,11 +225,11 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
         // the descriptor's low 14 bits hold the address / 16: adding an offset never carries out of them
         const uint64_t desc = desc0 + (uint64_t)(sa * (C::kActUnitBytes >> 4));
         const uint32_t a_tmem = tmem + C::kTmemA + r * 64;
-        tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, C::kIdesc, accumulate);
+        tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, idesc, accumulate);
         tc_commit(a_empty + 8 * (n & 1));               // unit 0's stage may be refilled when these MMAs are done
         mbar_wait_bounded<20>(a_full + 8 * (sa + 1), aphase, p.status, dead);
         tc_fence_after();
-        tc_mma_unit<kStepDesc>(d_tmem, a_tmem + 32, desc + (uint64_t)(C::kActUnitBytes >> 4), C::kIdesc, 1u);
+        tc_mma_unit<kStepDesc>(d_tmem, a_tmem + 32, desc + (uint64_t)(C::kActUnitBytes >> 4), idesc, 1u);
         tc_commit(done + 8 * r);                        // unit 1's stage and the operand slot are free then
         accumulate = 1;
         if (++blk == kb || n + 1 == nseg) {             // the slice ends
@@ -249,18 +252,19 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   } else if (warp >= C::kDeqBase) {
     // ================================================================== dequantisers (warps kDeqBase..)
     // thread = weight column = TMEM lane; team t expands the segments n = t, t + T, ... of the CTA
-    // and writes out rows [t NT/T, (t+1) NT/T) of every slice's accumulator tile
-    constexpr int RPT = C::kRowsPerTeam, CH = C::kChunk;
+    // and writes out its half (in multiples of 16 rows) of every slice's accumulator tile
+    constexpr int CH = C::kChunk;
     const int team = (warp - C::kDeqBase) >> 2;
     const int quarter = warp & 3;                    // the TMEM lanes this warp may touch
     const int c = quarter * 32 + lane;               // weight column inside the strip
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
     grid_dependency_wait();                          // the waits below depend, through the MMAs, on the previous kernel's output
     const uint32_t a_base = lane_base + C::kTmemA;
-    const uint32_t d_base = lane_base + C::kTmemD + team * RPT;
     const uint32_t lds_lo = c * 32 + 16 * ((c >> 2) & 1);          // words 0..3 of the column; words 4..7 at ^ 16
     const int strip_first = B0 / kb;
-    const int row0 = team * RPT;
+    const int team0_rows = (nt / 2 + CH - 1) / CH * CH;
+    const int row0 = team == 0 ? 0 : team0_rows, team_rows = team == 0 ? team0_rows : nt - team0_rows;     // both > 0: nt > 128
+    const uint32_t d_base = lane_base + C::kTmemD + row0;
 
     struct Slice {
       int strip_lin, strip, tile_row0;      // strip_lin: the VIRTUAL strip (row tile x strip)
@@ -270,7 +274,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       Slice sl;
       const int real = strip_lin % nstrips;
       sl.strip_lin = strip_lin;
-      sl.tile_row0 = (strip_lin / nstrips) * NT;
+      sl.tile_row0 = (strip_lin / nstrips) * nt;
       sl.is6 = real >= geo.strips4;
       sl.strip = sl.is6 ? real - geo.strips4 : real;
       sl.group = !sl.is6 && geo.groups > 1;
@@ -369,10 +373,10 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       }
       unsigned long long* slot = slot_of(cta);
 #pragma unroll 1
-      for (int m0 = 0; m0 < RPT; m0 += CH) {
+      for (int m0 = 0; m0 < team_rows; m0 += CH) {
         float t[CH];
         tc_ld16(d_base + m0, t);
-        if (m0 + CH == RPT) {
+        if (m0 + CH == team_rows) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(d_read);          // this warp has read its part: with the others', the issuer may start the next slice
@@ -536,12 +540,12 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   }
 }
 
-using Wide256 = WideCfg<256, 2, 4, 4>;    // 256 + 4 x 64 = 512 TMEM columns
+using Wide256 = WideCfg<kWideTileRows, 2, 4, 4>;    // 256 + 4 x 64 = 512 TMEM columns
 
 template <class C>
 cudaError_t launch_wide(const MulParams& p_in, cudaStream_t stream, bool overlap) {
   alignas(64) CUtensorMap amap;
-  cudaError_t me = encode_activation_map(p_in.A, p_in.M, p_in.K, C::NT, &amap);
+  cudaError_t me = encode_activation_map(p_in.A, p_in.M, p_in.K, p_in.tile_rows, &amap);
   if (me != cudaSuccess) return me;
   MulParams p = p_in;
   alignas(64) OutMaps omaps = {};
@@ -682,19 +686,20 @@ cudaError_t encode_activation_segment_map(const half* A, int M, int K, int box_r
   return cudaSuccess;
 }
 
-int wide_rows_per_pass() { return 256; }   // the widest tile
-
-// rows of the MMA tile used for `rows` rows of A
-int wide_tile_rows(int rows) { (void)rows; return 256; }
-
-size_t wide_scratch_bytes(int ctas, int rows) {
-  return kEpochWords * sizeof(unsigned int) + (size_t)ctas * wide_tile_rows(rows) * kStripCols * sizeof(unsigned long long);
+// `rows` (> 128) rows of A go into as few tiles as hold them, all of the same height (a multiple of 16, above 128)
+int wide_row_tiles(int rows) { return (rows + kWideTileRows - 1) / kWideTileRows; }
+int wide_tile_rows(int rows) {
+  const int tiles = wide_row_tiles(rows);
+  return ((rows + tiles - 1) / tiles + 15) / 16 * 16;
 }
 
-// Runs the GEMM for rows [0, p.M) in p.row_tiles tiles of `tile_rows` rows; the host dispatcher loops over larger M.
-cudaError_t launch_gemm_wide(const MulParams& p, int tile_rows, cudaStream_t stream) {
+size_t wide_scratch_bytes(int ctas) {
+  return kEpochWords * sizeof(unsigned int) + (size_t)ctas * kWideTileRows * kStripCols * sizeof(unsigned long long);
+}
+
+// Runs the GEMM for rows [0, p.M) in p.row_tiles tiles of p.tile_rows rows; the host dispatcher loops over larger M.
+cudaError_t launch_gemm_wide(const MulParams& p, cudaStream_t stream) {
   const bool overlap = tc5_get_overlap();
-  (void)tile_rows;                     // always 256: up to 128 rows go to the kernel of gemm_tc5.cu
   return launch_wide<Wide256>(p, stream, overlap);
 }
 

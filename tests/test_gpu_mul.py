@@ -366,6 +366,28 @@ def test_weights_written_by_the_gemm_in_front(m1, m2):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,k,n,qc", [
+    (129, 512, 1024, 128), (145, 384, 768, 256), (256, 4096, 512, 128),      # one tile of 144, 160 and 256 rows
+    (257, 512, 1024, 128), (288, 128, 2048, 256), (289, 2048, 768, -1),      # two of 144 and 160
+    (513, 640, 512, 512), (777, 1024, 1280, 32), (1025, 256, 768, 256),      # three of 176, four and five of 208
+    (2052, 16384, 256, 128), (2177, 16384, 512, 256),                        # a second launch of 4 rows (other kernel) and of 129
+])
+def test_heights_of_row_tiles(m, k, n, qc):
+    """The kernel for more than 128 rows cuts a launch's rows into tiles of one height, a multiple of 16; the last launch of
+    several may go to the other kernel.  Against fp32 products of the operands the kernels build."""
+    dev = _dev()
+    w = synth.make_layer(k, n, qc, 128, seed=m, keep_dequantized=False).to(dev)
+    a = synth.make_activations(m, k, m).to(dev)
+    c = torch.full((m + 1, n), 77.0, dtype=torch.float16, device=dev)
+    workspace = torch.zeros(n // 128 * 16 + 16, dtype=torch.int32, device=dev)
+    fm.mul(a, w.B, c[:m], w.s, workspace, qc, group_size=128, layout="b200")
+    ref = a.double() @ fm.dump_operands(w.B, w.s, k, n, qc, 128).double()
+    assert fm.device_status(dev) == 0
+    assert (torch.linalg.norm(c[:m].double() - ref, dim=1) / torch.linalg.norm(ref, dim=1)).max().item() <= TOL
+    assert bool((c[m] == 77.0).all())                                        # nothing is stored behind the last row
+
+
+@pytest.mark.gpu
 def test_gpu_weight_preparation_matches_host_bytes():
     """Quantise + cast + pack on the GPU gives the same packed words and scales as the host path."""
     dev = _dev()

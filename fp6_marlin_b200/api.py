@@ -479,6 +479,28 @@ def mul_fused(A, B, C, s, workspace, quant_cols=-1, *, epilogue="none", residual
         raise RuntimeError(f"fp6m_mul_fused failed with code {rc}")
 
 
+def gather_columns(c: torch.Tensor, src: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """``c.index_select(1, src) + bias`` (``c`` (M, N) fp16, ``src`` N column numbers, ``bias`` N values or None).  One kernel
+    for contiguous fp16 / int64 CUDA tensors of one device whose N is a multiple of 8; the torch operations for
+    anything else, and where autograd needs to see them."""
+    n = c.shape[1]
+    tensors = (c, src) if bias is None else (c, src, bias)
+    if (c.is_cuda and c.dtype == torch.float16 and c.is_contiguous() and n % 8 == 0 and src.dtype == torch.int64 and src.shape == (n,)
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.device == c.device and t.is_contiguous() for t in tensors)
+            and src.data_ptr() % 16 == 0
+            and (bias is None or (bias.dtype == torch.float16 and bias.shape == (n,) and bias.data_ptr() % 16 == 0))
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))):
+        y = torch.empty_like(c)
+        idx = c.device.index
+        rc = lib.fp6m_gather_columns(_ptr(c), _ptr(y), _ptr(src), 0 if bias is None else _ptr(bias), c.shape[0], n, idx,
+                                     _stream_handle(idx, c.device))
+        if rc:
+            raise RuntimeError(f"fp6m_gather_columns failed with code {rc}")
+        return y
+    c = c.index_select(1, src)
+    return c if bias is None else c + bias
+
+
 def dump_operands(B: torch.Tensor, s: torch.Tensor, k: int, n: int, quant_cols: int = -1, group_size: int = -1):
     """The fp16 matrix W_deq[k, n] that the GEMM kernels feed the tensor cores (b200 layout in)."""
     W = torch.zeros((k, n), dtype=torch.float16, device=B.device)

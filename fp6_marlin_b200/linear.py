@@ -53,9 +53,7 @@ class W46Linear(torch.nn.Module):
         c = torch.empty((a.shape[0], self.out_features), dtype=torch.float16, device=a.device)
         api.mul(a, self.B, c, self.s, self.workspace, self.quant_cols, group_size=self.group_size, layout="b200")
         if self.restore_order:
-            c = c.index_select(1, self.inverse_permutation)
-            if self.bias is not None:
-                c = c + self.bias
+            c = api.gather_columns(c, self.inverse_permutation, self.bias)
         elif self.bias is not None:
             c = c + self.bias.index_select(0, self.output_permutation)
         return c.reshape(*lead, self.out_features)

@@ -217,6 +217,11 @@ int fp6m_pack_b200_device(const void* q4, const void* c6, const void* s4, const 
 int fp6m_quantize_pack_b200_device(const void* w, int K, int N, int quant_cols, int group_size, void* B_out, void* s_out,
                                    int dev, void* stream, int* status_dev);
 
+/* y[m, f] = c[m, src[f]] (+ bias[f], one fp16 addition): puts the columns of an M x N row-major fp16 matrix into another
+ * order.  N a multiple of 8; y, src (int64) and bias (or null) 16-byte aligned; y must not overlap c.  An index outside
+ * 0..N-1 gives NaN.  The reference leaves the column order to its caller (fp6_marlin_cuda.cpp:93-122). */
+int fp6m_gather_columns(const void* c, void* y, const void* src, const void* bias, int M, int N, int dev, void* stream);
+
 /* Process-wide option, off by default; returns the previous setting (a negative argument only queries).
  * GEMMs of up to 128 rows are always launched with programmatic stream serialisation: such a GEMM sets itself up (and brings the first
  * lines of B into L2) while the kernel before it in the stream finishes, and reads and writes memory only after that

@@ -50,6 +50,7 @@ struct LaunchPlan {
   int tile;         // (most) rows of A per MMA tile
   int rows;         // rows of A per launch
   int ctas;         // grid of the first (largest) launch
+  int row_ctas;     // CTAs that the device offers (for the number of row tiles)
 };
 
 // `sms` <= 0: the largest grid any device can get (an upper bound for sizing buffers).
@@ -78,10 +79,11 @@ LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches =
   if (max_tiles > kMaxRowTiles) max_tiles = kMaxRowTiles;
   lp.rows = lp.wide ? lp.tile * max_tiles : lp.tile;
   const int launch_rows = M < lp.rows ? M : lp.rows;
-  const int row_tiles = lp.wide ? (launch_rows + lp.tile - 1) / lp.tile : 1;
   const int cap = lp.wide ? kMaxWideCtas : kMaxCtas;
   long long want = sms > 0 ? (long long)sms * (lp.wide ? 1 : tc5_ctas_per_sm(launch_rows)) : cap;
   int ctas = want < cap ? (int)want : cap;
+  const int row_tiles = lp.wide ? wide_row_tiles(launch_rows, geo, ctas) : 1;     // (more with a larger grid: without a device an upper bound)
+  lp.row_ctas = ctas;
   // at least ~16 units per CTA, also when that leaves SMs idle: a small GEMM split over every SM spends
   // its time in the split-K reduction (16 contributors per strip for N = 1024), not in streaming
   const long long total_units = (long long)row_tiles * (geo.strips4 + geo.strips6) * units_per_strip(geo);
@@ -217,8 +219,8 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     // its partials fit (half as many rows, two slots per CTA).
     const bool launch_wide = wide && p.M > kTc5MaxRows;
     const int launch_ctas = wide && !launch_wide ? std::min(ctas, plan_launches(p.M, p.geo, sms).ctas) : ctas;
-    p.row_tiles = launch_wide ? wide_row_tiles(p.M) : 1;
-    p.tile_rows = launch_wide ? wide_tile_rows(p.M) : 0;
+    p.row_tiles = launch_wide ? wide_row_tiles(p.M, p.geo, lp.row_ctas) : 1;
+    p.tile_rows = launch_wide ? wide_tile_rows(p.M, p.row_tiles) : 0;
     make_schedule(p.geo, launch_ctas, &p.sched, p.row_tiles);
     align_schedule_to_blocks(&p.sched);
     cudaError_t e = launch_wide ? launch_gemm_wide(p, static_cast<cudaStream_t>(stream)) : launch_gemm_tc5(p, static_cast<cudaStream_t>(stream));

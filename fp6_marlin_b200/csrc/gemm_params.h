@@ -78,8 +78,8 @@ cudaError_t encode_output_map(const half* base, int rows, int ld, CUtensorMap* m
 constexpr int kMaxWideCtas = 192;   // one CTA per SM
 constexpr int kMaxRowTiles = 32;    // 8192 rows of A per launch
 constexpr int kWideTileRows = 256;  // most rows of a tile
-int wide_row_tiles(int rows);
-int wide_tile_rows(int rows);
+int wide_row_tiles(int rows, const Geometry& geo, int ctas);
+int wide_tile_rows(int rows, int tiles);
 size_t wide_scratch_bytes(int ctas);
 cudaError_t launch_gemm_wide(const MulParams& p, cudaStream_t stream);
 

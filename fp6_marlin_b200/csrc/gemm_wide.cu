@@ -12,8 +12,7 @@
 //     8-row groups; a K step of 16 advances the descriptor by 32 bytes.  Rows beyond M are zero-filled
 //     by the copy engine.
 //   * Segments are whole 128-row blocks (two units); one thread issues all their MMAs.
-//   * The rows of a launch are cut into tiles of one height, the smallest multiple of 16 that needs no more tiles than 256
-//     would: the time of an MMA and of an activations copy goes with the rows (264 rows as 2 x 144 instead of 2 x 256: 4096 x 4096
+//   * The rows of a launch are cut into tiles of one height, a multiple of 16 (wide_row_tiles): the time of an MMA and of an activations copy goes with the rows (264 rows as 2 x 144 instead of 2 x 256: 4096 x 4096
 //     40.2 -> 30.3 us, K = N = 8192 78.8 -> 56.0, 4096 x 22016 85.3 -> 73.5; 777 rows as 4 x 208: 4096 x 22016 173 -> 167).
 // One CTA per SM: warp 0 weights producer, warp 1 activations producer, warp 2 MMA issuer (and owner of TMEM), warp 3
 // reads the launch epoch, then four dequantiser warps per team; teams take the segments in turn.
@@ -263,7 +262,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
     const uint32_t lds_lo = c * 32 + 16 * ((c >> 2) & 1);          // words 0..3 of the column; words 4..7 at ^ 16
     const int strip_first = B0 / kb;
     const int team0_rows = (nt / 2 + CH - 1) / CH * CH;
-    const int row0 = team == 0 ? 0 : team0_rows, team_rows = team == 0 ? team0_rows : nt - team0_rows;     // both > 0: nt > 128
+    const int row0 = team == 0 ? 0 : team0_rows, team_rows = team == 0 ? team0_rows : nt - team0_rows;     // both > 0: nt >= 48
     const uint32_t d_base = lane_base + C::kTmemD + row0;
 
     struct Slice {
@@ -686,12 +685,27 @@ cudaError_t encode_activation_segment_map(const half* A, int M, int K, int box_r
   return cudaSuccess;
 }
 
-// `rows` (> 128) rows of A go into as few tiles as hold them, all of the same height (a multiple of 16, above 128)
-int wide_row_tiles(int rows) { return (rows + kWideTileRows - 1) / kWideTileRows; }
-int wide_tile_rows(int rows) {
-  const int tiles = wide_row_tiles(rows);
-  return ((rows + tiles - 1) / tiles + 15) / 16 * 16;
+static int tile_height(int rows, int tiles) { return ((rows + tiles - 1) / tiles + 15) / 16 * 16; }
+
+// `rows` (> 128) rows of A go into tiles of one height, a multiple of 16: as few as hold them, and more where strips
+// would otherwise be shared by several of the `ctas` CTAs.  Another tile dequantises all weights once more, but leaves
+// fewer and lower partial tiles to exchange.  It pays up to 14 blocks per CTA, or up to 38 when the tiles stay high enough
+// (112 rows) for the MMAs to cover the dequantisers; measured, us with n / n + 1 (/ n + 2 ...) tiles, n the fewest:
+// 1024 x 4096 (1.7 blocks per CTA and tile) 256 rows 28 / 21 / 19 / 17, 512 rows 29 / 24 / 21; 4096 x 4096 (6.9) 129 rows 29 / 24 / 25,
+// 256 rows 42 / 27 / 29, 512 rows 41 / 36 / 34, 777 rows 42 / 44; 11008 x 4096 (18.6) 201 rows 65 / 54, 256 rows 73 / 56, 300 rows 62 / 66;
+// K = N = 8192 (28) 256 rows 55 / 62; 4096 x 12288, more than one strip per CTA with two tiles, 256 rows 42 / 46.
+int wide_row_tiles(int rows, const Geometry& geo, int ctas) {
+  const int strips = geo.strips4 + geo.strips6;
+  int tiles = (rows + kWideTileRows - 1) / kWideTileRows;
+  while (true) {
+    const int more = tiles + 1, height = tile_height(rows, more);
+    const long long blocks = (long long)more * strips * geo.k128;
+    const bool pays = blocks <= 14ll * ctas || (height >= 112 && blocks <= 38ll * ctas);
+    if (more > kMaxRowTiles || (long long)more * strips > ctas || height < 48 || !pays) return tiles;     // (both teams need rows)
+    tiles = more;
+  }
 }
+int wide_tile_rows(int rows, int tiles) { return tile_height(rows, tiles); }
 
 size_t wide_scratch_bytes(int ctas) {
   return kEpochWords * sizeof(unsigned int) + (size_t)ctas * kWideTileRows * kStripCols * sizeof(unsigned long long);

@@ -367,9 +367,11 @@ def test_weights_written_by_the_gemm_in_front(m1, m2):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,k,n,qc", [
-    (129, 512, 1024, 128), (145, 384, 768, 256), (256, 4096, 512, 128),      # one tile of 144, 160 and 256 rows
-    (257, 512, 1024, 128), (288, 128, 2048, 256), (289, 2048, 768, -1),      # two of 144 and 160
-    (513, 640, 512, 512), (777, 1024, 1280, 32), (1025, 256, 768, 256),      # three of 176, four and five of 208
+    (129, 512, 1024, 128), (145, 384, 768, 256), (256, 4096, 512, 128),
+    (257, 512, 1024, 128), (288, 128, 2048, 256), (289, 2048, 768, -1),
+    (513, 640, 512, 512), (777, 1024, 1280, 32), (1025, 256, 768, 256),
+    (129, 8192, 12288, 128), (777, 2048, 12288, 256),                        # one tile of 144 rows, four of 208
+    (129, 128, 256, 128), (300, 4096, 512, 64), (512, 1024, 1024, 128), (1000, 11008, 256, -1),   # more tiles than needed, of 48 rows and more
     (2052, 16384, 256, 128), (2177, 16384, 512, 256),                        # a second launch of 4 rows (other kernel) and of 129
 ])
 def test_heights_of_row_tiles(m, k, n, qc):

@@ -408,33 +408,35 @@ int fp6m_unpack_reference(const uint8_t* B_ref, const uint16_t* s_ref, int K, in
   const uint32_t* int4_words = reinterpret_cast<const uint32_t*>(B_ref);
   const uint32_t* fp6_two = int4_words + (size_t)K * n4 / 8;          // INT4 region is K*n4/2 bytes
   const uint32_t* fp6_four = fp6_two + (size_t)K * n6 / 16;
-  static const int nib_src[8] = {0, 2, 4, 6, 1, 3, 5, 7};             // nibble p holds value index
-  for (int kb = 0; kb < K / 16; ++kb) {
-    for (int ch = 0; ch < n4 / 64; ++ch)
-      for (int lane = 0; lane < 32; ++lane) {
-        const int g = lane >> 2, t = lane & 3;
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t word = int4_words[(((size_t)kb * (n4 / 64) + ch) * 32 + lane) * 4 + j];
-          for (int p = 0; p < 8; ++p) {
-            const int vi = nib_src[p], h = vi >> 2, v = vi & 3;
-            q4[(size_t)frag_row(kb, t, v) * n4 + frag_col(ch, j, h, g)] = (word >> (4 * p)) & 15u;
+  static constexpr int nib_src[8] = {0, 2, 4, 6, 1, 3, 5, 7};         // nibble p holds value index
+  parallel_for((size_t)K / 16, [=](size_t lo, size_t hi) {       // 16 rows of the codes each
+    for (int kb = (int)lo; kb < (int)hi; ++kb) {
+      for (int ch = 0; ch < n4 / 64; ++ch)
+        for (int lane = 0; lane < 32; ++lane) {
+          const int g = lane >> 2, t = lane & 3;
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t word = int4_words[(((size_t)kb * (n4 / 64) + ch) * 32 + lane) * 4 + j];
+            for (int p = 0; p < 8; ++p) {
+              const int vi = nib_src[p], h = vi >> 2, v = vi & 3;
+              q4[(size_t)frag_row(kb, t, v) * n4 + frag_col(ch, j, h, g)] = (word >> (4 * p)) & 15u;
+            }
           }
         }
-      }
-    for (int ch = 0; ch < n6 / 64; ++ch)
-      for (int lane = 0; lane < 32; ++lane) {
-        const int g = lane >> 2, t = lane & 3;
-        const size_t base = ((size_t)kb * (n6 / 64) + ch) * 32 + lane;
-        for (int j = 0; j < 4; ++j)
-          for (int h = 0; h < 2; ++h)
-            for (int v = 0; v < 4; ++v) {
-              const int by = kByteOfV[v];
-              const uint32_t lo = (fp6_four[base * 4 + j] >> (8 * by + (h == 0 ? 4 : 0))) & 15u;
-              const uint32_t hi = (fp6_two[base * 2 + (j >> 1)] >> (8 * by + 6 - (4 * (j & 1) + 2 * h))) & 3u;
-              c6[(size_t)frag_row(kb, t, v) * n6 + frag_col(ch, j, h, g)] = (uint8_t)((hi << 4) | lo);
-            }
-      }
-  }
+      for (int ch = 0; ch < n6 / 64; ++ch)
+        for (int lane = 0; lane < 32; ++lane) {
+          const int g = lane >> 2, t = lane & 3;
+          const size_t base = ((size_t)kb * (n6 / 64) + ch) * 32 + lane;
+          for (int j = 0; j < 4; ++j)
+            for (int h = 0; h < 2; ++h)
+              for (int v = 0; v < 4; ++v) {
+                const int by = kByteOfV[v];
+                const uint32_t lo = (fp6_four[base * 4 + j] >> (8 * by + (h == 0 ? 4 : 0))) & 15u;
+                const uint32_t hi = (fp6_two[base * 2 + (j >> 1)] >> (8 * by + 6 - (4 * (j & 1) + 2 * h))) & 3u;
+                c6[(size_t)frag_row(kb, t, v) * n6 + frag_col(ch, j, h, g)] = (uint8_t)((hi << 4) | lo);
+              }
+        }
+    }
+  });
   for (int i = 0; i < n4; ++i) s4[(i / 32) * 32 + ref_scale_perm(i % 32)] = s_ref[i];
   for (int i = 0; i < n6; ++i) s6[(i / 32) * 32 + ref_scale_perm(i % 32)] = s_ref[n4 + i];
   return FP6M_OK;

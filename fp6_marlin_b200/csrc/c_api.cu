@@ -54,7 +54,7 @@ struct LaunchPlan {
 };
 
 // `sms` <= 0: the largest grid any device can get (an upper bound for sizing buffers).
-LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches = -1) {
+LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches = -1, bool fewest_tiles = false) {
   LaunchPlan lp;
   // 129 to 256 rows are one tile of the other kernel - since that sums a shared strip where the strip starts and cuts its
   // tiles to the rows there are, faster on every layer measured than two launches of the kernel for up to 128 rows
@@ -82,8 +82,8 @@ LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches =
   const int cap = lp.wide ? kMaxWideCtas : kMaxCtas;
   long long want = sms > 0 ? (long long)sms * (lp.wide ? 1 : tc5_ctas_per_sm(launch_rows)) : cap;
   int ctas = want < cap ? (int)want : cap;
-  const int row_tiles = lp.wide ? wide_row_tiles(launch_rows, geo, ctas) : 1;     // (more with a larger grid: without a device an upper bound)
-  lp.row_ctas = ctas;
+  lp.row_ctas = fewest_tiles ? 0 : ctas;            // 0: no tile beyond those that hold the rows
+  const int row_tiles = lp.wide ? wide_row_tiles(launch_rows, geo, lp.row_ctas) : 1;     // (more with a larger grid: without a device an upper bound)
   // at least ~16 units per CTA, also when that leaves SMs idle: a small GEMM split over every SM spends
   // its time in the split-K reduction (16 contributors per strip for N = 1024), not in streaming
   const long long total_units = (long long)row_tiles * (geo.strips4 + geo.strips6) * units_per_strip(geo);
@@ -177,7 +177,9 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
   if ((long long)kMaxRowTiles * (p.geo.strips4 + p.geo.strips6) * units_per_strip(p.geo) > 0x3fffffff) return FP6M_ERR_PROB_SHAPE;
   // up to kTc5MaxRows rows (up to twice as many on some layers, in two launches): the kernel with fp32 group scaling;
   // more: the wide kernel, tiles of up to 256 rows, up to kMaxRowTiles tiles per launch
-  const LaunchPlan lp = plan_launches(M, p.geo, sms);
+  LaunchPlan lp = plan_launches(M, p.geo, sms);
+  // a caller's fixed scratch (fp6m_mul_static_scratch) may hold the partials of the fewest tiles only
+  if (scratch_bytes < scratch_bytes_of(lp)) lp = plan_launches(M, p.geo, sms, -1, true);
   const bool wide = lp.wide;
   const int tile = lp.tile, rows = lp.rows, ctas = lp.ctas;
   if (scratch_bytes < scratch_bytes_of(lp)) return FP6M_ERR_SCRATCH;

@@ -390,6 +390,26 @@ def test_heights_of_row_tiles(m, k, n, qc):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [200, 300])
+def test_static_scratch_takes_small_layers_with_many_rows(m):
+    """The 16 MiB scratch holds the partials of the fewest row tiles, not those of the plan with more of them."""
+    from fp6_marlin_b200 import _lib
+    dev = _dev()
+    k, n = 1024, 2048
+    w = synth.make_layer(k, n, 128, 128, seed=m, keep_dequantized=False).to(dev)
+    a = synth.make_activations(m, k, m).to(dev)
+    c = torch.zeros((m, n), dtype=torch.float16, device=dev)
+    workspace = torch.zeros(n // 128 * 16, dtype=torch.int32, device=dev)
+    assert _lib.lib.fp6m_mul_scratch_bytes(m, n, k, 128, 148) > 16 << 20
+    rc = _lib.lib.fp6m_mul_static_scratch(a.data_ptr(), w.B.data_ptr(), c.data_ptr(), w.s.data_ptr(), m, n, k, workspace.data_ptr(),
+                                          workspace.numel() * 4, 0, torch.cuda.current_stream().cuda_stream, -1, -1, -1, 16, 128, 128,
+                                          _lib.LAYOUT_B200, None)
+    assert rc == _lib.OK
+    ref = a.double() @ fm.dump_operands(w.B, w.s, k, n, 128, 128).double()
+    assert (torch.linalg.norm(c.double() - ref) / torch.linalg.norm(ref)).item() <= TOL
+
+
+@pytest.mark.gpu
 def test_gpu_weight_preparation_matches_host_bytes():
     """Quantise + cast + pack on the GPU gives the same packed words and scales as the host path."""
     dev = _dev()

@@ -304,9 +304,12 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
         store_column_rows<CH>(p, sl.tile_row0 + row0 + m0, sl.is6, sl.strip * kStripCols + c, out, writes);
         return;
       }
+      const int row_first = sl.tile_row0 + row0 + m0;
+      if (row_first >= p.M) return;                    // nothing of the block exists (uniform over the team): it takes no turn
       const uint32_t buf = my_stage + (uint32_t)(stage_turn & 1) * (16 * kStripCols * 2);
       ++stage_turn;
-      // the copy engine has read the rows this buffer held two blocks ago (only team thread 0 issues copies)
+      // The copy engine has read the rows this buffer held two turns ago: team thread 0 commits exactly one group per turn,
+      // empty when the rows leave by ordinary stores, so all groups but the latest include that turn's.
       if (team_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
       named_bar_sync(1 + team, 128);
 #pragma unroll
@@ -317,19 +320,18 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the copy engine reads what this thread wrote
       named_bar_sync(1 + team, 128);
       const int ncols = strip_cols(sl.is6 ? geo.n6 : geo.n4, sl.strip);
-      const int row_first = sl.tile_row0 + row0 + m0;
-      if (row_first >= p.M) return;                    // uniform over the team
       const int col_strip = (p.out.n_out == 0 ? (sl.is6 ? geo.n4 : 0) : (sl.is6 ? p.out.col6 : p.out.col4)) + sl.strip * kStripCols;
-      if (p.vec_rows == 2 && ncols == kStripCols) {
-        // a full strip: one asynchronous tensor store per output; the team goes on at once
-        if (team_tid == 0) {
+      // a full strip: one asynchronous tensor store per output; the team goes on at once
+      const bool tensor_store = p.vec_rows == 2 && ncols == kStripCols;
+      if (team_tid == 0) {
+        if (tensor_store) {
           const int n_maps = p.out.n_out == 0 ? 1 : p.out.n_out;
 #pragma unroll 1
           for (int q = 0; q < n_maps; ++q) tma_store_rows(&omaps.m[q], buf, col_strip, row_first);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-        return;
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
+      if (tensor_store) return;
       const int g = team_tid & 15;                     // eight columns of the strip
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
@@ -348,7 +350,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
           }
         }
       }
-      // (the buffer is not written again before the barrier at the top of the block after next)
+      // (the buffer is not written again before the barrier at the top of the next turn)
     };
     // before the team leaves: its asynchronous stores have been performed
     auto drain_stores = [&]() {

@@ -56,17 +56,18 @@ struct LaunchPlan {
 // `sms` <= 0: the largest grid any device can get (an upper bound for sizing buffers).
 LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches = -1, bool fewest_tiles = false) {
   LaunchPlan lp;
-  // 129 to 256 rows are one tile of the other kernel - since that sums a shared strip where the strip starts and cuts its
-  // tiles to the rows there are, faster on every layer measured than two launches of the kernel for up to 128 rows
-  // (us at 129 / 201 / 256 rows, two launches -> one: 4096 x 4096 34 / 46 / 47 -> 29 / 37 / 42, 4096 x 12288 43 / 54 / 55 -> 33 / 38 / 42,
-  // 11008 x 4096 58 / 67 / 68 -> 42 / 51 / 57, 4096 x 22016 58 / 74 / 73 -> 44 / 50 / 54, 1024 x 4096 28 / 36 / 36 -> 21 / 25 / 29).
-  // Except between 24 and 32 blocks per CTA: there two launches are the plan that fp6m_mul_launches is documented and
-  // tested to report (K = N = 8192), although one would be faster there too (60 / 70 / 66 -> 40 / 46 / 50 us).
+  // 129 to 256 rows on a layer with up to 48 blocks per CTA: two launches of the kernel for up to 128 rows.  It multiplies the
+  // fp32 sums by the INT4 group scales; the other kernel rounds every scaled weight to fp16 first, which costs bits
+  // (INT4 columns against 64-bit sums, K = 1024 to 11008: relative error 2.07e-4 here, 2.67e-4 there; with the rounding of
+  // the result alone 2.07e-4).  One launch of the other kernel would be faster (201 rows of 4096 x 4096 in W46Linear: 33 us
+  // instead of 49).  On larger layers one launch is the plan: there two take longer even than one with 256-row tiles (K = N =
+  // 16384, 111 blocks per CTA, 4 %).  Layers with one scale per column, on which both kernels agree, keep the plan of the
+  // others, so that fp6m_mul_launches needs no group size.
   // `two_launches`: -1 decides here, 0 / 1 force (sizing a buffer for either).
   bool two = false;
   if (M > kTc5MaxRows && M <= 2 * kTc5MaxRows) {
-    const long long blocks = (long long)(geo.strips4 + geo.strips6) * geo.k128, ctas = sms > 0 ? sms : 148;
-    two = two_launches < 0 ? blocks > 24 * ctas && blocks <= 32 * ctas : two_launches != 0;
+    const long long blocks = (long long)(geo.strips4 + geo.strips6) * geo.k128;
+    two = two_launches < 0 ? blocks <= 48ll * (sms > 0 ? sms : 148) : two_launches != 0;
   }
   lp.wide = M > kTc5MaxRows && !two;
   lp.tile = lp.wide ? kWideTileRows : tc5_tile_rows(M < kTc5MaxRows ? M : kTc5MaxRows);

@@ -390,7 +390,30 @@ def test_heights_of_row_tiles(m, k, n, qc):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("m", [200, 300])
+@pytest.mark.parametrize("m,k,n", [(128, 2048, 2048), (129, 1024, 1024), (201, 4096, 4096), (256, 11008, 4096), (200, 8192, 8192)])
+@pytest.mark.parametrize("gs", [128, -1])
+def test_scales_in_fp32_up_to_256_rows(m, k, n, gs):
+    """Up to 128 rows, and up to 256 on layers of at most 48 blocks per CTA, scales are applied to fp32 sums: against 64-bit
+    sums of the exact codes and scales there is little but the rounding of the result to fp16.  (The fp32 sums add some
+    1e-6 of the result, 1 % of its rounding; weights rounded to fp16 would make it 29 % larger.)"""
+    dev = _dev()
+    qc = 256
+    w = fm.make_w46_weight(synth.make_weight_fp16(k, n, qc, seed=m), qc, gs, keep_dequantized=False, quant_device=dev)
+    q4, c6, s4, s6 = fm.unpack_b200(w.B, w.s, k, n, qc, gs)
+    s4 = s4.double().repeat_interleave(128, 0) if gs > 0 else s4.double()
+    w64 = torch.cat([(q4.double() - 8) * s4, fm.decode_fp6(c6).double() * s6.double()], dim=1).to(dev)
+    a = synth.make_activations(m, k, m).to(dev)
+    c = torch.zeros((m, n), dtype=torch.float16, device=dev)
+    workspace = torch.zeros(n // 128 * 16, dtype=torch.int32, device=dev)
+    fm.mul(a, w.B, c, w.s, workspace, qc, group_size=gs, layout="b200")
+    ref = a.double() @ w64
+    for cols in (slice(0, n - qc), slice(n - qc, n)):
+        rounding = torch.linalg.norm(ref[:, cols].half().double() - ref[:, cols])
+        assert (torch.linalg.norm(c[:, cols].double() - ref[:, cols]) / rounding).item() <= 1.05
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [257, 300])
 def test_static_scratch_takes_small_layers_with_many_rows(m):
     """The 16 MiB scratch holds the partials of the fewest row tiles, not those of the plan with more of them."""
     from fp6_marlin_b200 import _lib

@@ -15,6 +15,7 @@ from __future__ import annotations
 import weakref
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import lib
@@ -479,24 +480,35 @@ def mul_fused(A, B, C, s, workspace, quant_cols=-1, *, epilogue="none", residual
         raise RuntimeError(f"fp6m_mul_fused failed with code {rc}")
 
 
+def _kernel_address(t: torch.Tensor):
+    """Address of the memory of `t`, or None where a kernel must not stand in for torch operations: a tensor with a
+    forward-mode tangent, or one that a function transform (vmap, jvp, grad) wraps and that has no memory of its own."""
+    try:
+        address = t.data_ptr()
+    except RuntimeError:
+        return None
+    return None if forward_ad.unpack_dual(t).tangent is not None else address
+
+
 def gather_columns(c: torch.Tensor, src: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """``c.index_select(1, src) + bias`` (``c`` (M, N) fp16, ``src`` N column numbers, ``bias`` N values or None).  One kernel
     for contiguous fp16 / int64 CUDA tensors of one device whose N is a multiple of 8; the torch operations for
-    anything else, and where autograd needs to see them."""
+    anything else, and where derivatives or function transforms need to see them.  The kernel writes NaN for a column
+    number outside 0..N-1, on which ``index_select`` stops with a device-side assertion."""
     n = c.shape[1]
     tensors = (c, src) if bias is None else (c, src, bias)
-    if (c.is_cuda and c.dtype == torch.float16 and c.is_contiguous() and n % 8 == 0 and src.dtype == torch.int64 and src.shape == (n,)
+    if (c.is_cuda and c.dtype == torch.float16 and n % 8 == 0 and src.dtype == torch.int64 and src.shape == (n,)
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.device == c.device and t.is_contiguous() for t in tensors)
-            and src.data_ptr() % 16 == 0
-            and (bias is None or (bias.dtype == torch.float16 and bias.shape == (n,) and bias.data_ptr() % 16 == 0))
+            and (bias is None or (bias.dtype == torch.float16 and bias.shape == (n,)))
             and not (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))):
-        y = torch.empty_like(c)
-        idx = c.device.index
-        rc = lib.fp6m_gather_columns(_ptr(c), _ptr(y), _ptr(src), 0 if bias is None else _ptr(bias), c.shape[0], n, idx,
-                                     _stream_handle(idx, c.device))
-        if rc:
-            raise RuntimeError(f"fp6m_gather_columns failed with code {rc}")
-        return y
+        at = [_kernel_address(t) for t in tensors]
+        if None not in at and not any(address % 16 for address in at[1:]):
+            y = torch.empty_like(c)
+            idx = c.device.index
+            rc = lib.fp6m_gather_columns(at[0], _ptr(y), at[1], 0 if bias is None else at[2], c.shape[0], n, idx, _stream_handle(idx, c.device))
+            if rc:
+                raise RuntimeError(f"fp6m_gather_columns failed with code {rc}")
+            return y
     c = c.index_select(1, src)
     return c if bias is None else c + bias
 

@@ -603,6 +603,25 @@ static EncodeTiledFn encode_tiled() {
   return fn;
 }
 
+// A map of fp16 data whose elements outside read as zero.  The encoder is a driver call and needs a current context, which a
+// thread that has made no other CUDA call does not have: cudaGetDevice binds none, so the first attempt fails there.
+static cudaError_t encode_f16(CUtensorMap* map, int rank, const half* base, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                              CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
+  EncodeTiledFn encode = encode_tiled();
+  if (!encode) return cudaErrorNotSupported;
+  const cuuint32_t elem[3] = {1, 1, 1};
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<half*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+      return cudaSuccess;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaSetDevice(dev);       // binds the device's primary context to the thread
+    if (e != cudaSuccess) return e;
+  }
+  return cudaErrorInvalidValue;
+}
+
 // The last few tensor maps of the calling thread: a decode loop calls with the same activation buffer again
 // and again, and encoding a map costs a driver call.  (A map depends on the pointer and the shape only.)
 namespace {
@@ -637,17 +656,12 @@ thread_local MapCache g_map_cache;
 cudaError_t encode_activation_map(const half* A, int M, int K, int box_rows, CUtensorMap* map) {
   const MapKey mk = {A, M, K, box_rows, 2};
   if (g_map_cache.find(mk, map)) return cudaSuccess;
-  EncodeTiledFn encode = encode_tiled();
-  if (!encode) return cudaErrorNotSupported;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
   const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<half*>(A), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return cudaErrorInvalidValue;
-  g_map_cache.put(mk, *map);
-  return cudaSuccess;
+  const cudaError_t e = encode_f16(map, 2, A, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+  if (e == cudaSuccess) g_map_cache.put(mk, *map);
+  return e;
 }
 
 // An output (C, or a rank's full-width output) as an `ld` x `rows` fp16 tensor; one box = 128 columns x 16 rows,
@@ -655,17 +669,12 @@ cudaError_t encode_activation_map(const half* A, int M, int K, int box_rows, CUt
 cudaError_t encode_output_map(const half* base, int rows, int ld, CUtensorMap* map) {
   const MapKey mk = {base, rows, ld, 16, 4};
   if (g_map_cache.find(mk, map)) return cudaSuccess;
-  EncodeTiledFn encode = encode_tiled();
-  if (!encode) return cudaErrorNotSupported;
   const cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
   const cuuint32_t box[2] = {(cuuint32_t)kStripCols, 16};
-  const cuuint32_t elem[2] = {1, 1};
-  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<half*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return cudaErrorInvalidValue;
-  g_map_cache.put(mk, *map);
-  return cudaSuccess;
+  const cudaError_t e = encode_f16(map, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+  if (e == cudaSuccess) g_map_cache.put(mk, *map);
+  return e;
 }
 
 // A as a 64 x M x K/64 tensor (K a multiple of 64): one box = 64 halves x `box_rows` rows x 2 units = the
@@ -674,17 +683,12 @@ cudaError_t encode_output_map(const half* base, int rows, int ld, CUtensorMap* m
 cudaError_t encode_activation_segment_map(const half* A, int M, int K, int box_rows, CUtensorMap* map) {
   const MapKey mk = {A, M, K, box_rows, 3};
   if (g_map_cache.find(mk, map)) return cudaSuccess;
-  EncodeTiledFn encode = encode_tiled();
-  if (!encode) return cudaErrorNotSupported;
   const cuuint64_t dims[3] = {64, (cuuint64_t)M, (cuuint64_t)(K / 64)};
   const cuuint64_t strides[2] = {(cuuint64_t)K * 2, 128};
   const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 2};
-  const cuuint32_t elem[3] = {1, 1, 1};
-  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<half*>(A), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return cudaErrorInvalidValue;
-  g_map_cache.put(mk, *map);
-  return cudaSuccess;
+  const cudaError_t e = encode_f16(map, 3, A, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+  if (e == cudaSuccess) g_map_cache.put(mk, *map);
+  return e;
 }
 
 static int tile_height(int rows, int tiles) { return ((rows + tiles - 1) / tiles + 15) / 16 * 16; }

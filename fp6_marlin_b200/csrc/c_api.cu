@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 
@@ -23,14 +24,14 @@ int cuda_fail(cudaError_t e, const char* where) {
 }
 
 int sm_count(int dev) {
-  static int cached[64] = {};
+  static std::atomic<int> cached[64] = {};
   if (dev < 0 || dev >= 64) return 0;
-  if (!cached[dev]) {
-    int n = 0;
+  int n = cached[dev];
+  if (!n) {
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     cached[dev] = n;
   }
-  return cached[dev];
+  return n;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -285,7 +286,7 @@ int fp6m_mul_static_scratch(const void* A, const void* B, void* C, const void* s
                             void* workspace, size_t workspace_bytes, int dev, void* stream,
                             int thread_k, int thread_n, int sms, int max_par,
                             int quant_cols, int group_size, int layout, int* status_dev) {
-  static void* scratch_of_device[64] = {};
+  static std::atomic<void*> scratch_of_device[64] = {};
   if (dev < 0 || dev >= 64) return FP6M_ERR_BAD_ARG;
   if (!scratch_of_device[dev]) {
     DeviceGuard guard(dev);                 // the symbol has one instance per device: ask with `dev` current

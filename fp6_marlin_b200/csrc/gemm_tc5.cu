@@ -66,6 +66,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "device_utils.cuh"
@@ -826,12 +827,12 @@ using Tc5Rows64Ordered = Tc5Cfg<64, 10, 4, 2, false>;
 using Tc5Rows128 = Tc5Cfg<128, 6, 4, 2, true, 2>;
 using Tc5Rows128Ordered = Tc5Cfg<128, 6, 4, 2, false, 2>;
 
-bool g_overlap_launches = false;
-bool g_ordered_sums = false;
+std::atomic<bool> g_overlap_launches{false};
+std::atomic<bool> g_ordered_sums{false};
 
 template <class C>
 cudaError_t launch_tc5(const MulParams& p, cudaStream_t stream) {
-  static bool configured[64] = {};
+  static std::atomic<bool> configured[64] = {};       // threads that find it false set the same attribute
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {

@@ -35,6 +35,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "device_utils.cuh"
 #include "fp6m_layout.h"
 #include "gemm_params.h"
@@ -561,7 +563,7 @@ cudaError_t launch_wide(const MulParams& p_in, cudaStream_t stream, bool overlap
     if (ok) p.vec_rows = 2;
   }
 
-  static bool configured[64] = {};
+  static std::atomic<bool> configured[64] = {};       // threads that find it false set the same attribute
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
@@ -588,18 +590,16 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// The driver's tensor-map encoder, looked up once through the runtime (no link against libcuda).
+// The driver's tensor-map encoder, looked up once through the runtime (no link against libcuda).  Several threads may make
+// the first call: the others wait for the one that looks it up.
 static EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
     void* sym = nullptr;
     cudaDriverEntryPointQueryResult res;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &res) == cudaSuccess &&
-        res == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(sym);
-  }
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &res) != cudaSuccess || res != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<EncodeTiledFn>(sym);
+  }();
   return fn;
 }
 

@@ -55,3 +55,12 @@ def run_from_threads(warm_up):
 def test_first_call_of_a_thread():
     """A thread that has made no CUDA call has no current context, which the driver's tensor-map encoder needs."""
     run_from_threads(warm_up=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("attempt", range(3))
+def test_first_calls_of_a_process_from_several_threads(attempt):
+    """The tensor-map encoder, kernel attributes and multiprocessor counts are looked up on first use."""
+    program = "import sys; sys.path[:0] = ['.', 'tests']; import test_gpu_first_calls as t; t.run_from_threads(warm_up=False); print('ok')"
+    run = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and run.stdout.strip().endswith("ok"), run.stdout[-2000:] + run.stderr[-2000:]

@@ -14,7 +14,7 @@ _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("FP6M_LIB") or os.path.join(_PKG_DIR, "libfp6m.so")
 
 OK, ERR_PROB_SHAPE, ERR_KERN_SHAPE, ERR_VALUE_RANGE, ERR_BAD_ARG = 0, 1, 2, 3, 4
-ERR_WORKSPACE, ERR_SCRATCH, ERR_CUDA, ERR_TIMEOUT = 5, 6, 7, 8
+ERR_WORKSPACE, ERR_SCRATCH, ERR_CUDA, ERR_TIMEOUT, ERR_NO_MEMORY = 5, 6, 7, 8, 9
 LAYOUT_REFERENCE, LAYOUT_B200 = 0, 1
 EPILOGUE_NONE, EPILOGUE_SILU_MUL, EPILOGUE_RESIDUAL = 0, 1, 2
 

@@ -245,6 +245,8 @@ def repack_from_reference(B_ref: torch.Tensor, s_ref: torch.Tensor, k: int, n: i
     rc = lib.fp6m_repack_from_reference(_ptr(src), _ptr(sc), k, n, quant_cols, _ptr(B), _ptr(s))
     if rc == _lib.ERR_PROB_SHAPE:
         raise ValueError("repack_from_reference: k must be a multiple of 16 and both regions multiples of 64 columns")
+    if rc == _lib.ERR_NO_MEMORY:
+        raise MemoryError("repack_from_reference: host memory ran out")
     if rc:
         raise RuntimeError(f"fp6m_repack_from_reference failed with code {rc}")
     return B.to(dev), s.to(dev)

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -71,20 +72,23 @@ inline uint16_t half_mul(uint16_t a, uint16_t b) {
   return float_to_half_bits(half_bits_to_float(a) * half_bits_to_float(b));
 }
 
+// Runs body(lo, hi), which must not throw, over [0, n) on up to 16 threads, the calling one among them.  Where the system has
+// no further thread (or no memory for its stack) the calling thread does the rest: callers are C entries, out of
+// which no exception may pass.
 template <typename F>
 void parallel_for(size_t n, F&& body) {
-  unsigned hw = std::thread::hardware_concurrency();
-  size_t threads = std::min<size_t>(hw ? hw : 1, 16);
-  if (n < 64 || threads <= 1) { body(0, n); return; }
-  threads = std::min(threads, n);
-  std::vector<std::thread> pool;
-  size_t chunk = (n + threads - 1) / threads;
-  for (size_t t = 0; t < threads; ++t) {
-    size_t lo = t * chunk, hi = std::min(n, lo + chunk);
-    if (lo >= hi) break;
-    pool.emplace_back([=, &body] { body(lo, hi); });
+  constexpr size_t kMaxThreads = 16;
+  const unsigned hw = std::thread::hardware_concurrency();
+  const size_t threads = n < 64 ? 1 : std::min<size_t>(hw ? hw : 1, kMaxThreads);
+  const size_t chunk = (n + threads - 1) / threads;
+  std::thread pool[kMaxThreads];
+  size_t started = 0, lo = 0;
+  try {
+    for (; lo + chunk < n; lo += chunk, ++started) pool[started] = std::thread([=, &body] { body(lo, lo + chunk); });
+  } catch (const std::exception&) {
   }
-  for (auto& th : pool) th.join();
+  body(lo, n);
+  for (size_t t = 0; t < started; ++t) pool[t].join();
 }
 
 // ---- FP6 E3M2 ---------------------------------------------------------------------------------
@@ -118,13 +122,15 @@ inline bool fp6_encode(uint16_t h, uint8_t* code) {
 //
 // The code of every half, 0x80 for those that have none (and 0x80 & 63 = code 0 in their place).
 const uint8_t* fp6_code_table() {
-  static const std::vector<uint8_t> table = [] {
-    std::vector<uint8_t> t(1 << 16, 0);
-    for (int h = 0; h < (1 << 16); ++h)
-      if (!fp6_encode((uint16_t)h, &t[h])) t[h] = 0x80;
-    return t;
-  }();
-  return table.data();
+  struct Table {
+    uint8_t of[1 << 16];
+    Table() {
+      for (int h = 0; h < (1 << 16); ++h)
+        if (!fp6_encode((uint16_t)h, &of[h])) of[h] = 0x80;
+    }
+  };
+  static const Table table;
+  return table.of;
 }
 
 // Exact value of a code as fp16 bits: `s 00eee mm 00000000` times 2^12 (weight_prepacking.cpp:199-212).
@@ -180,13 +186,12 @@ int fp6m_quantize_fp6(const uint16_t* w, uint8_t* out, size_t rows, size_t cols)
 
 int fp6m_encode_fp6(const uint16_t* w, uint8_t* codes, size_t count) {
   if (!w || !codes) return FP6M_ERR_BAD_ARG;
-  std::vector<int> bad(1, 0);
-  int* bad_flag = bad.data();
-  parallel_for(count, [=](size_t lo, size_t hi) {
+  std::atomic<int> bad(0);
+  parallel_for(count, [=, &bad](size_t lo, size_t hi) {
     for (size_t i = lo; i < hi; ++i)
-      if (!fp6_encode(w[i], &codes[i])) { *bad_flag = 1; codes[i] = 0; }
+      if (!fp6_encode(w[i], &codes[i])) { bad.store(1, std::memory_order_relaxed); codes[i] = 0; }
   });
-  return bad[0] ? FP6M_ERR_VALUE_RANGE : FP6M_OK;
+  return bad.load() ? FP6M_ERR_VALUE_RANGE : FP6M_OK;
 }
 
 int fp6m_prepack_fp6(const uint8_t* fp6, uint8_t* out, size_t n, size_t k) {
@@ -446,8 +451,16 @@ int fp6m_repack_from_reference(const uint8_t* B_ref, const uint16_t* s_ref, int 
                                uint8_t* B_out, uint16_t* s_out) {
   if (K <= 0 || N <= 0 || qc > N) return FP6M_ERR_BAD_ARG;
   const int n6 = qc < 0 ? 0 : qc, n4 = N - n6;
-  std::vector<uint8_t> q4((size_t)K * n4), c6((size_t)K * n6);
-  std::vector<uint16_t> s4(n4), s6(n6);
+  std::vector<uint8_t> q4, c6;
+  std::vector<uint16_t> s4, s6;
+  try {
+    q4.resize((size_t)K * n4);
+    c6.resize((size_t)K * n6);
+    s4.resize(n4);
+    s6.resize(n6);
+  } catch (const std::exception&) {
+    return FP6M_ERR_NO_MEMORY;
+  }
   int rc = fp6m_unpack_reference(B_ref, s_ref, K, N, qc, q4.data(), c6.data(), s4.data(), s6.data());
   if (rc) return rc;
   return fp6m_pack_b200(q4.data(), c6.data(), s4.data(), s6.data(), K, N, qc, -1, B_out, s_out);

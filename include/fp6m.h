@@ -26,7 +26,8 @@ enum {
   FP6M_ERR_WORKSPACE = 5,    /* workspace smaller than the reference demands (fp6_marlin_cuda.cpp:62-63) */
   FP6M_ERR_SCRATCH = 6,      /* scratch buffer smaller than fp6m_mul_scratch_bytes() */
   FP6M_ERR_CUDA = 7,         /* a CUDA runtime call failed; see fp6m_last_cuda_error() */
-  FP6M_ERR_TIMEOUT = 8       /* device status word: a bounded wait inside a kernel ran out */
+  FP6M_ERR_TIMEOUT = 8,      /* device status word: a bounded wait inside a kernel ran out */
+  FP6M_ERR_NO_MEMORY = 9     /* host memory ran out (fp6m_repack_from_reference) */
 };
 
 enum { FP6M_LAYOUT_REFERENCE = 0, FP6M_LAYOUT_B200 = 1 };

@@ -1,9 +1,13 @@
 """The host codec on every half and on every code under scales of all kinds, against the oracle's restatement."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 import fp6_marlin_b200 as fm
+from conftest import ROOT
 from oracle import formats as F
 
 
@@ -50,3 +54,36 @@ def test_prepacking_places_every_code(n, k):
     B, s = fm.repack_from_reference(packed, torch.ones(n, dtype=torch.float16), k, n, n)
     _, c6, _, _ = fm.unpack_b200(B, s, k, n, n, -1)
     assert np.array_equal(c6.numpy(), _codes(stream, n, k).T)
+
+
+def test_no_thread_and_no_memory():
+    """Without room for the stack of a thread (or for the codes that re-tiling keeps) the host functions run on the calling thread
+    (or report it): no exception leaves a C entry, which would end the process."""
+    program = """
+import resource, torch
+import fp6_marlin_b200 as fm
+from fp6_marlin_b200 import _lib
+
+k, n = 256, 512
+torch.manual_seed(0)
+x, s = fm.fake_quantize_fp6(torch.randn((k, n)).half())
+B, ref = torch.randint(-2**31, 2**31, (k * n * 3 // 16,)).int(), torch.rand(n).half()
+q4, s4 = torch.randint(0, 16, (k, n), dtype=torch.uint8), torch.rand((k // 128, n)).half()
+def work():
+    codes = fm.quantize(x)
+    stream = codes.view(n, k * 3 // 16)
+    return [codes, fm.prepacking(stream), fm.dequantize(stream, s), fm.encode_fp6(x), *fm.pack_b200(q4, None, s4, None, k, n, -1, 128),
+            *fm.repack_from_reference(B, ref, k, n, n)]
+expect = work()
+big_k, big_n = 16384, 8192
+big = torch.zeros(big_k * big_n // 8, dtype=torch.int32)
+out, out_s = torch.zeros(fm.b200_sizes(big_k, big_n)[0], dtype=torch.int32), torch.zeros(big_n).half()
+pages = int(open('/proc/self/statm').read().split()[0])
+resource.setrlimit(resource.RLIMIT_AS, (pages * resource.getpagesize() + (4 << 20),) * 2)
+assert all(torch.equal(a, b) for a, b in zip(work(), expect))
+rc = _lib.lib.fp6m_repack_from_reference(big.data_ptr(), out_s.data_ptr(), big_k, big_n, -1, out.data_ptr(), out_s.data_ptr())
+assert rc == _lib.ERR_NO_MEMORY, rc
+print("ok")
+"""
+    run = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0 and run.stdout.strip() == "ok", run.stdout + run.stderr

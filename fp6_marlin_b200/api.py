@@ -264,7 +264,8 @@ def schedule(k: int, n: int, quant_cols: int = -1, group_size: int = -1, ctas: i
 
 def launch_plan(m: int, n: int, k: int, quant_cols: int = -1, sms: int = 148):
     """How `mul` cuts the shape into kernel launches on a device with `sms` multiprocessors: (number of
-    launches, True if the kernel for more than 128 rows runs)."""
+    launches, True if the kernel for more than 128 rows runs).  For ``group_size=128``; with one scale per column 129 to 256
+    rows are one launch of that kernel on every layer."""
     import ctypes
     many = ctypes.c_int(0)
     launches = lib.fp6m_mul_launches(m, n, k, quant_cols, sms, ctypes.byref(many))

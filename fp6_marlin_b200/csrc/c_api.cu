@@ -57,18 +57,20 @@ struct LaunchPlan {
 // `sms` <= 0: the largest grid any device can get (an upper bound for sizing buffers).
 LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches = -1, bool fewest_tiles = false) {
   LaunchPlan lp;
-  // 129 to 256 rows on a layer with up to 48 blocks per CTA: two launches of the kernel for up to 128 rows.  It multiplies the
-  // fp32 sums by the INT4 group scales; the other kernel rounds every scaled weight to fp16 first, which costs bits
-  // (INT4 columns against 64-bit sums, K = 1024 to 11008: relative error 2.07e-4 here, 2.67e-4 there; with the rounding of
-  // the result alone 2.07e-4).  One launch of the other kernel would be faster (201 rows of 4096 x 4096 in W46Linear: 33 us
-  // instead of 49).  On larger layers one launch is the plan: there two take longer even than one with 256-row tiles (K = N =
-  // 16384, 111 blocks per CTA, 4 %).  Layers with one scale per column, on which both kernels agree, keep the plan of the
-  // others, so that fp6m_mul_launches needs no group size.
+  // 129 to 256 rows on a layer with INT4 group scales and up to 48 blocks per CTA: two launches of the kernel for up to 128 rows.
+  // It multiplies the fp32 sums by the group scales; the other kernel rounds every scaled weight to fp16 first, which costs
+  // bits (INT4 columns against 64-bit sums, K = 1024 to 11008: relative error 2.07e-4 here, 2.67e-4 there; with the rounding
+  // of the result alone 2.07e-4).  One launch of the other kernel is faster and is the plan of layers without group scales, on
+  // which the errors of both kernels agree to five digits (us at 129 / 201 / 256 rows, two launches -> one: 4096 x 4096
+  // 33 / 44 / 44 -> 24 / 27 / 27, 4096 x 12288 41 / 52 / 52 -> 31 / 36 / 39, K = N = 8192 47 / 59 / 59 -> 39 / 45 / 49, 11008 x 4096
+  // 43 / 56 / 56 -> 40 / 42 / 43, 1024 x 4096 26 / 35 / 36 -> 17, 4096 x 22016 56 / 69 / 74 -> 43 / 49 / 54), and of larger layers,
+  // where two launches take longer even than one with 256-row tiles (K = N = 16384, 111 blocks per CTA, 4 %).
   // `two_launches`: -1 decides here, 0 / 1 force (sizing a buffer for either).
   bool two = false;
   if (M > kTc5MaxRows && M <= 2 * kTc5MaxRows) {
     const long long blocks = (long long)(geo.strips4 + geo.strips6) * geo.k128;
-    two = two_launches < 0 ? blocks <= 48ll * (sms > 0 ? sms : 148) : two_launches != 0;
+    const bool group_scales = geo.groups > 1 && geo.strips4 > 0;
+    two = two_launches < 0 ? group_scales && blocks <= 48ll * (sms > 0 ? sms : 148) : two_launches != 0;
   }
   lp.wide = M > kTc5MaxRows && !two;
   lp.tile = lp.wide ? kWideTileRows : tc5_tile_rows(M < kTc5MaxRows ? M : kTc5MaxRows);
@@ -119,8 +121,8 @@ size_t fp6m_mul_scratch_bytes(int M, int N, int K, int quant_cols, int sms) {
   }
   const int qc = quant_cols < 0 ? 0 : (quant_cols > N ? N : quant_cols);
   const Geometry geo = make_geometry(K, N, qc, 128);
-  if (sms <= 0 && M > kTc5MaxRows && M <= 2 * kTc5MaxRows) {
-    // no device given: enough for either way of cutting 129 to 256 rows into launches
+  if (M > kTc5MaxRows && M <= 2 * kTc5MaxRows) {
+    // neither the group size is given here nor always a device: enough for either way of cutting 129 to 256 rows into launches
     const size_t a = scratch_bytes_of(plan_launches(M, geo, sms, 0)), b = scratch_bytes_of(plan_launches(M, geo, sms, 1));
     return a > b ? a : b;
   }

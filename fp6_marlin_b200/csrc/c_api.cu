@@ -190,7 +190,6 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
   p.B = static_cast<const uint8_t*>(B);
   p.S = static_cast<const half*>(s);
   p.N = N; p.K = K;
-  p.counters = static_cast<int*>(workspace);
   p.epochs = static_cast<unsigned int*>(scratch);
   p.partials = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) + kEpochWords * sizeof(unsigned int));
   p.status = status_dev;

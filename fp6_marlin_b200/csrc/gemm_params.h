@@ -43,7 +43,6 @@ struct MulParams {
   int M, N, K;
   int row_tiles;        // wide kernel: tiles of rows of A covered by this launch (virtual strips = row_tiles x strips)
   Geometry geo;
-  int* counters;        // one zero-initialised int per strip (the caller's workspace; left untouched)
   unsigned int* epochs;            // scratch header: [0] launch epoch, [1] CTAs of this launch that have read it
   unsigned long long* partials;    // split-K slots (scratch): {fp32 value, epoch tag} per 64-bit word
   int* status;          // optional device status word

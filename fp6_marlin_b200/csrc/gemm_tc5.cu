@@ -643,13 +643,11 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
       const int n_next = n + T;
       stage += T;
       if (stage >= S) { stage -= S; wphase ^= 1; }
-      bool was6 = sp.is6;
       while (n_next >= sp.n_end && sp.n_end < nseg) sp = open_strip(++s);
       if (n_next < nseg) {
         mbar_wait(w_full + 8 * stage, wphase, ws);
         load_words(sp, stage, w);
       }
-      (void)was6;
       FP6M_TRACE_EVENT(trace, 18, n);
       tc_wait_st();
       FP6M_TRACE_EVENT(trace, 19, n);

@@ -302,7 +302,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       float out[CH];
 #pragma unroll
       for (int i = 0; i < CH; ++i) out[i] = v[i] * col_scale;
-      if (!p.vec_rows || CH != 16) {
+      if (!p.vec_rows) {
         store_column_rows<CH>(p, sl.tile_row0 + row0 + m0, sl.is6, sl.strip * kStripCols + c, out, writes);
         return;
       }

@@ -329,8 +329,9 @@ def _device_buffers(device: torch.device, shape=None, stream=None):
 
 def set_launch_overlap(enable: bool) -> bool:
     """Process-wide switch (off by default): GEMMs may read their weights and scales before the kernel in front
-    of them in the stream has finished; returns the previous setting.  (Their set-up always overlaps that kernel; A,
-    C, the scratch and - with the switch off - the weights are only touched after it has completed.)  Only turn it on
+    of them in the stream has finished; returns the previous setting.  (The set-up of GEMMs of up to 128 rows always overlaps
+    that kernel, that of others with the switch on; A, C, the scratch and - with the switch off - the weights are only
+    touched after it has completed.)  Only turn it on
     when the kernel preceding a GEMM in its stream does not write that GEMM's weights or scales."""
     return bool(lib.fp6m_set_launch_overlap(1 if enable else 0))
 

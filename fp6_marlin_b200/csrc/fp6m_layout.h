@@ -130,8 +130,8 @@ FP6M_HD int int4_nibble_pos(int i) { return (i & 1) ? 4 + (i >> 1) : (i >> 1); }
 // ---------------------------------------------------------------------------------------------
 // Stripe schedule.  Units are ordered strip-major (INT4 strips, then FP6 strips), rows fastest,
 // and weighted by their cost (unit_cost: 8 per INT4 unit, 11 per FP6 unit).  CTA c owns the units
-// [bound[c], bound[c+1]); a strip that is shared by several CTAs is reduced in fp32 by the last
-// of them to finish.  Replaces the reference's static INT4/FP6 SM split and its stripe
+// [bound[c], bound[c+1]); a strip that is shared by several CTAs is summed in fp32 by one of them:
+// the one in which it ends (kernel for up to 128 rows) or starts (kernel for more).  Replaces the reference's static INT4/FP6 SM split and its stripe
 // arithmetic (fp6_marlin_cuda_kernel.cu:308-408).
 // ---------------------------------------------------------------------------------------------
 struct Schedule {
@@ -193,9 +193,10 @@ inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_ti
   const long long total_cost = (long long)row_tiles * ups * ((long long)kInt4UnitCost * g.strips4 + (long long)kFp6UnitCost * g.strips6);
   out->ctas = ctas;
   out->total_units = total_units;
-  // A CTA whose range starts inside a strip and reaches the strip's end reduces that strip at its own end
-  // (the kernel for up to 128 rows): such CTAs get `kReducerPenalty` cost units (one segment) less work than
-  // the others - measured 1 to 2 % on the steps of the Llama-2 layers; two or four segments less are no better.
+  // In the kernel for up to 128 rows a CTA whose range starts inside a strip and reaches the strip's end reduces that strip
+  // at its own end: such CTAs get `kReducerPenalty` cost units (one segment) less work than the others - measured 1 to 2 % on
+  // the steps of the Llama-2 layers; two or four segments less are no better.  (The kernel for more than 128 rows, which sums a
+  // strip where it starts, gets the same shares when it has one tile of rows.)
   // Which CTAs they are depends on the boundaries, so the shares are settled in a few rounds.
   constexpr int kReducerPenalty = 16;
   double share[kMaxCtas];
@@ -234,8 +235,7 @@ inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_ti
   }
 }
 
-// Moves every inner boundary to a whole block (an even unit): the kernel for up to 128 rows works on
-// 128-row blocks.  The number of units per strip is even, so strips and the total stay aligned.
+// Moves every inner boundary to a whole block (an even unit): both kernels work on 128-row blocks.  The number of units per strip is even, so strips and the total stay aligned.
 inline void align_schedule_to_blocks(Schedule* s) {
   for (int c = 1; c < s->ctas; ++c) s->bound[c] = (s->bound[c] + 1) & ~1;
 }

@@ -15,7 +15,7 @@ constexpr int kThreads = 128, kRows = 4;
 // one region keep their order, so a warp's two-byte reads fall into few lines, and the result leaves as 16-byte stores.
 // Latency-bound at the sizes of a decode step or a short prompt (3 x 67 rows of 4096 features: 3.3 MB): one launch, started
 // while the kernel in front of it finishes, in place of an index_select and an addition: that W46Linear call with a bias
-// took 60.1 us with the GEMM at 46 and takes 43.3 with the GEMM at 37 to 38.
+// takes 49 us with the GEMM (two launches) at 44, and took 60 with the two torch operations and the GEMM at 46.
 __global__ void __launch_bounds__(kThreads) gather_columns_kernel(const half* __restrict__ c, half* __restrict__ y, const long long* __restrict__ src,
                                                                   const half* __restrict__ bias, int M, int N) {
   const int col = (blockIdx.x * kThreads + threadIdx.x) * 8;

@@ -1,19 +1,21 @@
-// W(4&6)A16 GEMM on tcgen05 + TMEM for 129 to 256 rows of A per pass (up to 128 rows: gemm_tc5.cu).
+// W(4&6)A16 GEMM on tcgen05 + TMEM for more than 128 rows of A (up to 128 rows, and on layers with group scales up to 256:
+// gemm_tc5.cu).
 //
 // As in the kernel for up to 128 rows (gemm_tc5.cu) the product is computed transposed: the 128 weight
 // columns of a strip are the M dimension of tcgen05.mma (one TMEM lane per column), the rows of A its
-// N dimension (128 or 256), the dequantised weights the A operand in TENSOR MEMORY.  Differences:
+// N dimension (a tile's height), the dequantised weights the A operand in TENSOR MEMORY.  Differences:
 //   * The INT4 group scale is multiplied into the operand - fp16(q - 8) * s_g with one fp16 rounding,
 //     bit for bit the dequantised weight of the reference's rule (test.py:98) - so ONE accumulator
 //     tile collects a whole slice of K and is read back once per slice, not once per scale group.
 //     Per-channel INT4 scales and FP6 scales (times 4096) are applied to the fp32 sums, as before.
-//   * The activations come by tiled TMA: one copy per 64-row unit brings NT rows x 64 halves (128-byte
+//   * The activations come by tiled TMA: one copy per 64-row unit brings a tile's rows x 64 halves (128-byte
 //     rows, 128-byte swizzle) - the K-major swizzled operand layout of tcgen05 with 1024 bytes between
 //     8-row groups; a K step of 16 advances the descriptor by 32 bytes.  Rows beyond M are zero-filled
 //     by the copy engine.
 //   * Segments are whole 128-row blocks (two units); one thread issues all their MMAs.
-//   * The rows of a launch are cut into tiles of one height, a multiple of 16 (wide_row_tiles): the time of an MMA and of an activations copy goes with the rows (264 rows as 2 x 144 instead of 2 x 256: 4096 x 4096
-//     40.2 -> 30.3 us, K = N = 8192 78.8 -> 56.0, 4096 x 22016 85.3 -> 73.5; 777 rows as 4 x 208: 4096 x 22016 173 -> 167).
+//   * The rows of a launch are cut into tiles of one height, a multiple of 16 from 48 to 256 (wide_row_tiles): the time of an
+//     MMA and of an activations copy goes with the rows (264 rows as 2 x 144 instead of 2 x 256: 4096 x 4096 40.2 -> 30.3 us,
+//     K = N = 8192 78.8 -> 56.0, 4096 x 22016 85.3 -> 73.5; 777 rows as 4 x 208: 4096 x 22016 173 -> 167).
 // One CTA per SM: warp 0 weights producer, warp 1 activations producer, warp 2 MMA issuer (and owner of TMEM), warp 3
 // reads the launch epoch, then four dequantiser warps per team; teams take the segments in turn.
 //
@@ -22,7 +24,8 @@
 // all but 190 of them the issuer's own: 764 for eight MMAs, the rest bookkeeping, three commits and three waits.  With
 // whole blocks, counters in place of a walk and two commits per segment, and with the slices written out only when
 // the operands of the next slice already wait in tensor memory (before, the pipe drained at every strip's end):
-// K = N = 16384 at M = 4096 2201 -> 1888 us (1165 TFLOP/s), 4096 x 22016 at M = 777 208 -> 179 us.
+// K = N = 16384 at M = 4096 2201 -> 1888 us in that comparison (1915 to 1950 in later runs on other GPUs), 4096 x 22016 at
+// M = 777 208 -> 179 us.
 // Split-K between CTAs uses tagged words as in gemm_tc5.cu, but the CTA in which a strip STARTS sums it: the slice is that CTA's
 // last, so its own sums never leave the chip and the next CTA's partial has long been stored.  (When the CTA in which
 // the strip ends did it, after its last segment, the reduction took 32,000 cycles, a tenth of the kernel at 4096 x 22016 and
@@ -696,10 +699,12 @@ static int tile_height(int rows, int tiles) { return ((rows + tiles - 1) / tiles
 // `rows` (> 128) rows of A go into tiles of one height, a multiple of 16: as few as hold them, and more where strips
 // would otherwise be shared by several of the `ctas` CTAs.  Another tile dequantises all weights once more, but leaves
 // fewer and lower partial tiles to exchange.  It pays up to 14 blocks per CTA, or up to 38 when the tiles stay high enough
-// (112 rows) for the MMAs to cover the dequantisers; measured, us with n / n + 1 (/ n + 2 ...) tiles, n the fewest:
-// 1024 x 4096 (1.7 blocks per CTA and tile) 256 rows 28 / 21 / 19 / 17, 512 rows 29 / 24 / 21; 4096 x 4096 (6.9) 129 rows 29 / 24 / 25,
-// 256 rows 42 / 27 / 29, 512 rows 41 / 36 / 34, 777 rows 42 / 44; 11008 x 4096 (18.6) 201 rows 65 / 54, 256 rows 73 / 56, 300 rows 62 / 66;
-// K = N = 8192 (28) 256 rows 55 / 62; 4096 x 12288, more than one strip per CTA with two tiles, 256 rows 42 / 46.
+// (112 rows) for the MMAs to cover the dequantisers; measured on layers with one scale per column, us with n / n + 1 / n + 2 / n + 3
+// tiles, n the fewest: 1024 x 4096 (1.7 blocks per CTA and tile) 256 rows 29 / 21 / 19 / 17, 512 rows 29 / 25 / 21 / 21; 4096 x 4096 (6.9) 129
+// rows 29 / 24 / 25 / 29, 256 rows 42 / 27 / 28 / 29, 512 rows 40 / 35 / 33 / 39, 777 rows 39 / 43; 8192 x 4096 and 4096 x 8192 (13.8) 201 rows
+// 54 / 41 / 43 and 39 / 33 / 41, 300 rows 42 / 49 and 400 rows 39 / 47; 11008 x 4096 (18.6) 201 rows 50 / 42 / 49, 256 rows 56 / 43 / 49, 300 rows
+// 46 / 51; K = N = 8192 (28) 256 rows 52 / 50, 300 rows 53 / 68; 4096 x 22016 (37) 200 rows 50 / 66; 4096 x 12288, more than one strip per
+// CTA with two tiles, 256 rows 42 / 45.
 int wide_row_tiles(int rows, const Geometry& geo, int ctas) {
   const int strips = geo.strips4 + geo.strips6;
   int tiles = (rows + kWideTileRows - 1) / kWideTileRows;

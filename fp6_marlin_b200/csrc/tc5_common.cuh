@@ -1,6 +1,6 @@
 // Device-side pieces shared by the tcgen05 GEMM kernels: programmatic-dependent-launch controls,
 // tcgen05 / TMEM wrappers, gpu-scope relaxed accesses for the tagged split-K slots, the launch
-// epoch, the in-register expanders and the walk over a CTA's units.
+// epoch and the in-register expanders.
 #pragma once
 #ifndef FP6M_PARTIAL_STORE_MODE
 #define FP6M_PARTIAL_STORE_MODE 0
@@ -18,11 +18,11 @@ namespace fp6m {
 constexpr int kStageW = 12288;          // packed words of one block: up to 2 x (4096 four-bit + 2048 two-bit)
 
 // ---- programmatic dependent launch ---------------------------------------------------------------
-// launch_dependents: the next kernel of the stream may start launching (it runs its set-up and
-// prefetches weights while this one finishes).  grid_dependency_wait: returns once every kernel this
-// one depends on has completed and its writes are visible; without a programmatic dependency both
-// are no-ops.  Everything that earlier kernels may have written (A, C, the scratch) is only touched
-// after the wait; the weights and scales are read before it.
+// launch_dependents: the next kernel of the stream may start launching (it runs its set-up and brings the first weights into
+// L2 while this one finishes).  grid_dependency_wait: returns once every kernel this one depends on has completed and
+// its writes are visible; without a programmatic dependency both are no-ops.  What earlier kernels may have written is
+// only touched after the wait: A, C, the scratch, and the weights and scales too unless the caller's switch says that
+// the kernel in front does not write them.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -376,14 +376,16 @@ def test_weights_written_by_the_gemm_in_front(m1, m2):
 ])
 def test_heights_of_row_tiles(m, k, n, qc):
     """The kernel for more than 128 rows cuts a launch's rows into tiles of one height, a multiple of 16; the last launch of
-    several may go to the other kernel.  Against fp32 products of the operands the kernels build."""
+    several may go to the other kernel.  (129 to 256 rows are its own with one scale per column.)  Against 64-bit products of
+    the operands the kernels build."""
     dev = _dev()
-    w = synth.make_layer(k, n, qc, 128, seed=m, keep_dequantized=False).to(dev)
+    gs = -1 if m <= 256 else 128
+    w = synth.make_layer(k, n, qc, gs, seed=m, keep_dequantized=False).to(dev)
     a = synth.make_activations(m, k, m).to(dev)
     c = torch.full((m + 1, n), 77.0, dtype=torch.float16, device=dev)
     workspace = torch.zeros(n // 128 * 16 + 16, dtype=torch.int32, device=dev)
-    fm.mul(a, w.B, c[:m], w.s, workspace, qc, group_size=128, layout="b200")
-    ref = a.double() @ fm.dump_operands(w.B, w.s, k, n, qc, 128).double()
+    fm.mul(a, w.B, c[:m], w.s, workspace, qc, group_size=gs, layout="b200")
+    ref = a.double() @ fm.dump_operands(w.B, w.s, k, n, qc, gs).double()
     assert fm.device_status(dev) == 0
     assert (torch.linalg.norm(c[:m].double() - ref, dim=1) / torch.linalg.norm(ref, dim=1)).max().item() <= TOL
     assert bool((c[m] == 77.0).all())                                        # nothing is stored behind the last row
@@ -391,13 +393,13 @@ def test_heights_of_row_tiles(m, k, n, qc):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,k,n", [(128, 2048, 2048), (129, 1024, 1024), (201, 4096, 4096), (256, 11008, 4096), (200, 8192, 8192)])
-@pytest.mark.parametrize("gs", [128, -1])
-def test_scales_in_fp32_up_to_256_rows(m, k, n, gs):
-    """Up to 128 rows, and up to 256 on layers of at most 48 blocks per CTA, scales are applied to fp32 sums: against 64-bit
+@pytest.mark.parametrize("gs,all_fp6", [(128, False), (-1, False), (128, True)])
+def test_scales_in_fp32_up_to_256_rows(m, k, n, gs, all_fp6):
+    """Up to 128 rows, and up to 256 on layers of at most 48 blocks per CTA or without INT4 group scales, scales are applied to fp32 sums: against 64-bit
     sums of the exact codes and scales there is little but the rounding of the result to fp16.  (The fp32 sums add some
     1e-6 of the result, 1 % of its rounding; weights rounded to fp16 would make it 29 % larger.)"""
     dev = _dev()
-    qc = 256
+    qc = n if all_fp6 else 256
     w = fm.make_w46_weight(synth.make_weight_fp16(k, n, qc, seed=m), qc, gs, keep_dequantized=False, quant_device=dev)
     q4, c6, s4, s6 = fm.unpack_b200(w.B, w.s, k, n, qc, gs)
     s4 = s4.double().repeat_interleave(128, 0) if gs > 0 else s4.double()
@@ -407,7 +409,7 @@ def test_scales_in_fp32_up_to_256_rows(m, k, n, gs):
     workspace = torch.zeros(n // 128 * 16, dtype=torch.int32, device=dev)
     fm.mul(a, w.B, c, w.s, workspace, qc, group_size=gs, layout="b200")
     ref = a.double() @ w64
-    for cols in (slice(0, n - qc), slice(n - qc, n)):
+    for cols in (slice(0, n - qc), slice(n - qc, n))[int(all_fp6):]:
         rounding = torch.linalg.norm(ref[:, cols].half().double() - ref[:, cols])
         assert (torch.linalg.norm(c[:, cols].double() - ref[:, cols]) / rounding).item() <= 1.05
 

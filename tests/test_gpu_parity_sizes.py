@@ -70,8 +70,8 @@ def test_compute_bound_geometry_with_several_launches(qc):
 
 
 def test_one_ragged_256_row_tile_on_a_large_layer():
-    """129 to 256 rows run in the kernel for more than 128 rows only on a layer with many blocks per CTA (on a
-    smaller one two launches of the other kernel are faster): K = 16384, N = 7424 has 58 x 128 blocks.  Checked on
+    """129 to 256 rows of a layer with group scales run in the kernel for more than 128 rows only with many blocks per CTA (on a
+    smaller one two launches of the other kernel, which keeps the scales in fp32): K = 16384, N = 7424 has 58 x 128 blocks.  Checked on
     four strips of columns (first, middle and last INT4 strip, the FP6 strips) against the oracle."""
     dev = _dev()
     k, n, qc, gs = 16384, 7424, 256, 128

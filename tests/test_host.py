@@ -277,7 +277,7 @@ def test_w46_linear_bookkeeping():
 def test_launch_plan_and_scratch_sizes():
     """How the host cuts M rows into launches (the reference's dispatcher loops over batches of rows as well,
     fp6_marlin_cuda_kernel.cu:917-948): one launch of the kernel for up to 128 rows; 129 to 256 rows as two launches
-    of it on a layer with at most 48 blocks per CTA, else one 256-row tile of the other kernel; more rows in launches
+    of it on a layer with group scales and at most 48 blocks per CTA, else one launch of the other kernel; more rows in launches
     whose activations stay within 64 MB.  The scratch size asked for without a device covers either plan."""
     sms = 148
     assert fm.launch_plan(0, 8192, 8192, 256, sms) == (0, False)

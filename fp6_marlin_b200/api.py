@@ -484,14 +484,12 @@ def mul_fused(A, B, C, s, workspace, quant_cols=-1, *, epilogue="none", residual
         raise RuntimeError(f"fp6m_mul_fused failed with code {rc}")
 
 
-def _kernel_address(t: torch.Tensor):
-    """Address of the memory of `t`, or None where a kernel must not stand in for torch operations: a tensor with a
-    forward-mode tangent, or one that a function transform (vmap, jvp, grad) wraps and that has no memory of its own."""
-    try:
-        address = t.data_ptr()
-    except RuntimeError:
-        return None
-    return None if forward_ad.unpack_dual(t).tangent is not None else address
+_PLAIN_TENSORS = (torch.Tensor, torch.nn.Parameter)
+
+
+def _has_tangent(tensors) -> bool:
+    """Whether one of the tensors carries a forward-mode derivative (which is only possible while a dual level is open)."""
+    return getattr(forward_ad, "_current_level", 0) >= 0 and any(forward_ad.unpack_dual(t).tangent is not None for t in tensors)
 
 
 def gather_columns(c: torch.Tensor, src: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
@@ -501,18 +499,26 @@ def gather_columns(c: torch.Tensor, src: torch.Tensor, bias: torch.Tensor | None
     number outside 0..N-1, on which ``index_select`` stops with a device-side assertion."""
     n = c.shape[1]
     tensors = (c, src) if bias is None else (c, src, bias)
-    if (c.is_cuda and c.dtype == torch.float16 and n % 8 == 0 and src.dtype == torch.int64 and src.shape == (n,)
-            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.device == c.device and t.is_contiguous() for t in tensors)
+    device = c.device
+    if (device.type == "cuda" and c.dtype == torch.float16 and n % 8 == 0 and src.dtype == torch.int64 and src.shape == (n,)
             and (bias is None or (bias.dtype == torch.float16 and bias.shape == (n,)))
-            and not (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))):
-        at = [_kernel_address(t) for t in tensors]
-        if None not in at and not any(address % 16 for address in at[1:]):
-            y = torch.empty_like(c)
-            idx = c.device.index
-            rc = lib.fp6m_gather_columns(at[0], _ptr(y), at[1], 0 if bias is None else at[2], c.shape[0], n, idx, _stream_handle(idx, c.device))
-            if rc:
-                raise RuntimeError(f"fp6m_gather_columns failed with code {rc}")
-            return y
+            and not (torch.is_grad_enabled() and (c.requires_grad or (bias is not None and bias.requires_grad)))):
+        addresses = []
+        for t in tensors:
+            if type(t) not in _PLAIN_TENSORS or t.device != device or not t.is_contiguous():
+                break
+            try:
+                addresses.append(t.data_ptr())
+            except RuntimeError:                # a wrapper of a function transform (vmap, jvp, grad) has no memory of its own
+                break
+        else:
+            if not any(address % 16 for address in addresses[1:]) and not _has_tangent(tensors):
+                y = torch.empty_like(c)
+                rc = lib.fp6m_gather_columns(addresses[0], _ptr(y), addresses[1], 0 if bias is None else addresses[2], c.shape[0], n, device.index,
+                                             _stream_handle(device.index, device))
+                if rc:
+                    raise RuntimeError(f"fp6m_gather_columns failed with code {rc}")
+                return y
     c = c.index_select(1, src)
     return c if bias is None else c + bias
 

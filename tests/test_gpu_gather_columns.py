@@ -59,6 +59,8 @@ def test_bias_under_function_transforms():
     many = torch.stack([bias, tangent, bias + tangent])
     mapped = torch.func.vmap(lambda b: api.gather_columns(c, src, b))(many)
     assert torch.equal(mapped, torch.stack([api.gather_columns(c, src, b) for b in many.unbind()]))
+    primal, pushed = torch.func.jvp(torch.func.vmap(lambda b: api.gather_columns(c, src, b)), (many,), (many,))
+    assert torch.equal(primal, mapped) and torch.equal(pushed, many[:, None].expand(3, 4, 64))
     grad = torch.func.grad(lambda b: api.gather_columns(c, src, b).float().sum())(bias)
     assert torch.equal(grad, torch.full_like(bias, 4.0))
 

@@ -13,6 +13,26 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ---- one thread of a warp -----------------------------------------------------------------------
+// The index of this thread's warp as a value the compiler knows to be the same in all its lanes.
+__device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// True in one lane of a converged warp, always the same one (tcgen05.commit tracks the MMAs of the thread that commits).
+// tcgen05.mma, tcgen05.commit and bulk copies take their operands from warp-wide uniform registers; behind elect.sync the
+// compiler knows that one thread issues them, behind `lane == 0` it does not.  Measured for four tcgen05.mma (128 x 16 x 16)
+// and a commit, cycles, alone / beside 8 / 16 warps of arithmetic: lane == 0 348 / 694 / 1217, elect.sync with operands that are
+// uniform to the compiler 44 / 52 / 60.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(one));
+  return one != 0;
+}
+
 // ---- mbarrier ---------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

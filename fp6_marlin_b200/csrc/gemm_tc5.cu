@@ -21,8 +21,8 @@
 //               units beyond K read as zero).
 //   warps 2-7   MMA issuers, two per dequantiser team (one per 64-row unit): four tcgen05.mma
 //               (kind::f16, fp32 accumulators in TMEM) per segment each, all accumulating into a tile
-//               the team zeroed, then a commit.  A thread needs ~140 cycles per MMA it issues while
-//               the tensor pipe needs ~32, so several threads have to issue side by side.  The two
+//               the team zeroed, then a commit (behind elect.sync, see elect_one: 11 to 15 cycles per MMA; behind `lane == 0`
+//               it was 175 beside busy teams, and K = N = 8192 at 16 / 64 rows took 13.8 / 20.8 us instead of 13.1 / 20.0).  The two
 //               commits of a segment tell the epilogue warps that the accumulator tile is ready and
 //               the team and the activations producer that operand slot and activation tile are free.
 //               Warp 2 owns the TMEM allocation; warp 7 also reads the launch epoch.
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
 
   if (warp == 0) {
     // ================================================================== weights producer, segments S..
-    if (lane == 0 && nseg > S) {
+    if (nseg > S) {
       int s = s_first, blk = blk_first + S;
       while (blk >= kb) { blk -= kb; ++s; }
       const uint8_t* src = p.B + segment_offset(geo, s, blk);
@@ -459,9 +459,12 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
       uint32_t phase = 0;                      // parity of the stage's previous use
       for (int n = S; n < nseg; ++n) {
         mbar_wait<200>(w_empty + 8 * stage, phase, ws);
-        mbar_arrive_expect_tx(w_full + 8 * stage, bytes + sbytes);
-        tma_load_1d_stream(smem0 + stage * kStageW, src, bytes, w_full + 8 * stage, policy);
-        if (sbytes) tma_load_1d_stream(smem0 + stage * kStageW + kStageScaleOff, ssrc, sbytes, w_full + 8 * stage, policy);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(w_full + 8 * stage, bytes + sbytes);
+          tma_load_1d_stream(smem0 + stage * kStageW, src, bytes, w_full + 8 * stage, policy);
+          if (sbytes) tma_load_1d_stream(smem0 + stage * kStageW + kStageScaleOff, ssrc, sbytes, w_full + 8 * stage, policy);
+        }
+        __syncwarp();
         FP6M_TRACE_EVENT(trace, 1, n);
         src += bytes;                          // blocks and strips follow one another without gaps
         ssrc += sbytes;                        // and so do the groups of a strip
@@ -476,13 +479,14 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
     }
   } else if (warp == 1) {
     // ================================================================== activations producer, segments R..
-    if (lane == 0 && nseg > R) {
+    if (nseg > R) {
       int blk = (blk_first + R) % kb;
       int r = 0;
       uint32_t phase = 0;                      // parity of the entry's previous use
       for (int n = R; n < nseg; ++n) {
         mbar_wait<200>(done + 8 * r, phase, ws);     // the MMAs that read this tile are done
-        load_activations(blk, r);
+        if (elect_one()) load_activations(blk, r);
+        __syncwarp();
         FP6M_TRACE_EVENT(trace, 5, n);
         if (++blk == kb) blk = 0;
         if (++r == R) { r = 0; phase ^= 1; }
@@ -495,9 +499,12 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
     // ring entry r and issues all eight MMAs of its segments.  The whole warp waits (warp-uniform control
     // flow); one fixed lane issues the tcgen05 instructions, so that the commit tracks the MMAs before it.
     // First of all, issuer i loads the activations of segment i.
-    const int mine = warp - 2;
-    if (lane == 0 && mine < R && mine < nseg) {
-      load_activations((blk_first + mine) % kb, mine);
+    // (warp index and tensor-memory base as values that are uniform to the compiler, see elect_one; only here: in the 128-row
+    // instance, uniform values that live through the whole kernel cost registers and spills)
+    const int mine = uniform_warp_index() - 2;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem, 0);
+    if (mine < R && mine < nseg) {
+      if (elect_one()) load_activations((blk_first + mine) % kb, mine);
       FP6M_TRACE_EVENT(trace, 5, mine);
     }
     __syncwarp();
@@ -513,11 +520,11 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
         if constexpr (C::kDecoupled) mbar_wait<32>(d_free + 8 * r, rphase, ws);      // the entry's accumulator tile is free and zero
         tc_fence_after();
         FP6M_TRACE_EVENT(trace, 6, n);
-        const uint32_t d_tmem = tmem + C::kTmemD + (C::kDecoupled ? n % C::kDRing : r) * NT;
-        const uint32_t a_tmem = tmem + C::kTmemA + r * 64 + unit * 32;
+        const uint32_t d_tmem = tmem_base + C::kTmemD + (C::kDecoupled ? n % C::kDRing : r) * NT;
+        const uint32_t a_tmem = tmem_base + C::kTmemA + r * 64 + unit * 32;
         // the descriptor's low 14 bits hold the address / 16: adding an offset never carries out of them
         const uint64_t desc = desc0 + (uint64_t)(r * (C::kActBytes >> 4));
-        if (lane == 0) {
+        if (elect_one()) {
           tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, C::kIdesc, 1u);
           tc_commit(done + 8 * r);
         }
@@ -531,15 +538,15 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
       const int r = mine;
       uint32_t rphase = 0;
       const uint64_t desc = wide_act_desc(act_base) + (uint64_t)(r * (C::kActBytes >> 4));
-      const uint32_t a_tmem = tmem + C::kTmemA + r * 64;
+      const uint32_t a_tmem = tmem_base + C::kTmemA + r * 64;
       for (int n = r; n < nseg; n += R) {
-        const uint32_t d_tmem = tmem + C::kTmemD + (C::kDecoupled ? n % C::kDRing : r) * NT;
+        const uint32_t d_tmem = tmem_base + C::kTmemD + (C::kDecoupled ? n % C::kDRing : r) * NT;
         mbar_wait<32>(ready + 8 * r, rphase, ws);
         mbar_wait<32>(act_full + 8 * r, rphase, ws);
         if constexpr (C::kDecoupled) mbar_wait<32>(d_free + 8 * r, rphase, ws);      // the entry's accumulator tile is free
         tc_fence_after();
         FP6M_TRACE_EVENT(trace, 6, n);
-        if (lane == 0) {
+        if (elect_one()) {
           tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, C::kIdesc, 0u);
           tc_mma_unit<kStepDesc>(d_tmem, a_tmem + 32, desc + (C::kActUnitBytes >> 4), C::kIdesc, 1u);
           tc_commit(done + 8 * r);

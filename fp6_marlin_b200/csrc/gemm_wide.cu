@@ -25,7 +25,9 @@
 // whole blocks, counters in place of a walk and two commits per segment, and with the slices written out only when
 // the operands of the next slice already wait in tensor memory (before, the pipe drained at every strip's end):
 // K = N = 16384 at M = 4096 2201 -> 1888 us in that comparison (1915 to 1950 in later runs on other GPUs), 4096 x 22016 at
-// M = 777 208 -> 179 us.
+// M = 777 208 -> 179 us.  The MMAs themselves are issued behind elect.sync with operands that are uniform to the compiler: four of
+// them and a commit then take 52 cycles of the issuing warp beside eight warps of arithmetic, behind `lane == 0` they took 694,
+// more than the 512 of the tensor pipe (K = N = 16384 at M = 1024 462 -> 412 us, 4096 x 22016 at M = 777 139 -> 133, GEMMs back to back).
 // Split-K between CTAs uses tagged words as in gemm_tc5.cu, but the CTA in which a strip STARTS sums it: the slice is that CTA's
 // last, so its own sums never leave the chip and the next CTA's partial has long been stored.  (When the CTA in which
 // the strip ends did it, after its last segment, the reduction took 32,000 cycles, a tenth of the kernel at 4096 x 22016 and
@@ -105,7 +107,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   const uint32_t ready = a_empty + 8 * 2, done = ready + 8 * R;
   const uint32_t slice_done = done + 8 * R, d_read = slice_done + 8, epoch_bar = d_read + 8;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp_index(), lane = tid & 31;
   // Ranges are handed out from the last to the first: a CTA that has to wait for the partials of higher ranges waits for
   // CTAs that were dispatched before it.
   const int cta = gridDim.x - 1 - blockIdx.x;
@@ -148,12 +150,12 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = misc[0];
+  const uint32_t tmem = __shfl_sync(0xffffffffu, misc[0], 0);      // uniform to the compiler
   bool dead = false;
 
   if (warp == 0) {
     // ================================================================== weights producer
-    if (lane == 0) {
+    {
       const uint64_t policy = make_evict_first_policy();
       int v = B0 / kb, blk = B0 - v * kb;
       int strip = v % nstrips;                         // the strip of the virtual strip
@@ -174,8 +176,11 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
       for (int n = 0; n < nseg; ++n) {
         if (n == S) grid_dependency_wait();            // the first S copies need nobody; from here on the teams must have made room
         mbar_wait_bounded<200>(w_empty + 8 * stage, phase ^ 1, p.status, dead);
-        mbar_arrive_expect_tx(w_full + 8 * stage, bytes);
-        tma_load_1d_stream(smem_u32(smem) + stage * kStageW, wsrc, bytes, w_full + 8 * stage, policy);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(w_full + 8 * stage, bytes);
+          tma_load_1d_stream(smem_u32(smem) + stage * kStageW, wsrc, bytes, w_full + 8 * stage, policy);
+        }
+        __syncwarp();
         wsrc += bytes;                                 // blocks of a strip are contiguous in HBM
         if (++stage == S) { stage = 0; phase ^= 1; }
         if (++blk == kb) {
@@ -189,7 +194,7 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
     // ================================================================== activations producer
     // Segment n's units go to the stages 2 (n % 2) and 2 (n % 2) + 1.  Unit 0's stage is free again when a_empty says that
     // the MMAs of segment n - 2 have read it, unit 1's when that segment is done altogether.
-    if (lane == 0) {
+    {
       int v = B0 / kb, blk = B0 - v * kb;
       grid_dependency_wait();                           // A may come from the previous kernel
       for (int n = 0; n < nseg; ++n) {
@@ -197,19 +202,26 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
         const int row0 = (v / nstrips) * nt;
         const uint32_t dst = smem_u32(act_base) + sa * C::kActUnitBytes;
         if (n >= 2) mbar_wait_bounded<100>(a_empty + 8 * (n & 1), ((n - 2) >> 1) & 1, p.status, dead);
-        mbar_arrive_expect_tx(a_full + 8 * sa, nt * 128);
-        tma_load_act_rows(dst, &amap, 2 * blk * kUnitRows, row0, a_full + 8 * sa);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(a_full + 8 * sa, nt * 128);
+          tma_load_act_rows(dst, &amap, 2 * blk * kUnitRows, row0, a_full + 8 * sa);
+        }
+        __syncwarp();
         if (n >= 2) mbar_wait_bounded<100>(done + 8 * ((n - 2) % R), ((n - 2) / R) & 1, p.status, dead);
-        mbar_arrive_expect_tx(a_full + 8 * (sa + 1), nt * 128);
-        tma_load_act_rows(dst + C::kActUnitBytes, &amap, (2 * blk + 1) * kUnitRows, row0, a_full + 8 * (sa + 1));
+        if (elect_one()) {
+          mbar_arrive_expect_tx(a_full + 8 * (sa + 1), nt * 128);
+          tma_load_act_rows(dst + C::kActUnitBytes, &amap, (2 * blk + 1) * kUnitRows, row0, a_full + 8 * (sa + 1));
+        }
+        __syncwarp();
         if (++blk == kb) { blk = 0; ++v; }
       }
     }
   } else if (warp == 2) {
     // ================================================================== MMA issuer
-    // One thread, so that the commits track its MMAs, with as little between the MMAs as possible: this thread was the
-    // kernel's serial chain (1741 cycles per segment at K = N = 16384, of which the tensor pipe needs 1024).
-    if (lane == 0) {
+    // One thread, so that the commits track its MMAs; the warp stays together around it (elect_one), with as little between
+    // the MMAs as possible: this warp was the kernel's serial chain (1741 cycles per segment at K = N = 16384, of which the
+    // tensor pipe needs 1024).
+    {
       // every bounded wait below depends on the activations, which the previous kernel of the stream may still be
       // writing: start them only when it has completed
       grid_dependency_wait();
@@ -229,15 +241,22 @@ w46_gemm_wide_kernel(const __grid_constant__ MulParams p, const __grid_constant_
         // the descriptor's low 14 bits hold the address / 16: adding an offset never carries out of them
         const uint64_t desc = desc0 + (uint64_t)(sa * (C::kActUnitBytes >> 4));
         const uint32_t a_tmem = tmem + C::kTmemA + r * 64;
-        tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, idesc, accumulate);
-        tc_commit(a_empty + 8 * (n & 1));               // unit 0's stage may be refilled when these MMAs are done
+        if (elect_one()) {
+          tc_mma_unit<kStepDesc>(d_tmem, a_tmem, desc, idesc, accumulate);
+          tc_commit(a_empty + 8 * (n & 1));             // unit 0's stage may be refilled when these MMAs are done
+        }
+        __syncwarp();
         mbar_wait_bounded<20>(a_full + 8 * (sa + 1), aphase, p.status, dead);
         tc_fence_after();
-        tc_mma_unit<kStepDesc>(d_tmem, a_tmem + 32, desc + (uint64_t)(C::kActUnitBytes >> 4), idesc, 1u);
-        tc_commit(done + 8 * r);                        // unit 1's stage and the operand slot are free then
+        const bool slice_ends = ++blk == kb || n + 1 == nseg;
+        if (elect_one()) {
+          tc_mma_unit<kStepDesc>(d_tmem, a_tmem + 32, desc + (uint64_t)(C::kActUnitBytes >> 4), idesc, 1u);
+          tc_commit(done + 8 * r);                      // unit 1's stage and the operand slot are free then
+          if (slice_ends) tc_commit(slice_done);
+        }
+        __syncwarp();
         accumulate = 1;
-        if (++blk == kb || n + 1 == nseg) {             // the slice ends
-          tc_commit(slice_done);
+        if (slice_ends) {
           blk = 0;
           accumulate = 0;
           ++slices;

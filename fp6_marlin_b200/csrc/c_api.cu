@@ -204,14 +204,10 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     for (int q = 0; q < out.n_out; ++q) ok = ok && aligned16(out.peer[q]);
     p.vec_rows = ok ? 1 : 0;
   }
-  // Expanding before the grid dependency resolves pays on a chain of launches when the next launch's CTAs get
-  // onto their SMs early enough: measured -10 % on a 4096 x 4096 layer (128 CTAs), -2 to -3 % with 32 to 128 rows
-  // or 19 blocks per CTA, +1 % (worse) with 28 blocks per CTA on every SM and 16 rows.
-  {
-    const long long blocks = (long long)(p.geo.strips4 + p.geo.strips6) * p.geo.k128;
-    p.weights_early = tc5_get_overlap() ? 1 : 0;
-    p.expand_early = (p.weights_early && !wide && (tile > 16 || blocks <= 20ll * ctas)) ? 1 : 0;
-  }
+  // The kernel for 33 to 128 rows may also expand its first segments before the grid dependency resolves (measured -2 to -3 %
+  // on a chain of launches).
+  p.weights_early = tc5_get_overlap() ? 1 : 0;
+  p.expand_early = (p.weights_early && !wide) ? 1 : 0;
 
   for (int m0 = 0; m0 < M; m0 += rows) {
     p.A = static_cast<const half*>(A) + (size_t)m0 * K;
@@ -226,10 +222,11 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     const int launch_ctas = wide && !launch_wide ? std::min(ctas, plan_launches(p.M, p.geo, sms).ctas) : ctas;
     p.row_tiles = launch_wide ? wide_row_tiles(p.M, p.geo, lp.row_ctas) : 1;
     p.tile_rows = launch_wide ? wide_tile_rows(p.M, p.row_tiles) : 0;
-    make_schedule(p.geo, launch_ctas, &p.sched, p.row_tiles);
+    make_schedule(p.geo, launch_ctas, &p.sched, p.row_tiles, !launch_wide && p.M <= kTeamMaxRows ? 0 : kReducerPenalty);
     align_schedule_to_blocks(&p.sched);
-    cudaError_t e = launch_wide ? launch_gemm_wide(p, static_cast<cudaStream_t>(stream)) : launch_gemm_tc5(p, static_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return cuda_fail(e, launch_wide ? "w46_gemm_wide launch" : "w46_gemm_tc5 launch");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e = launch_wide ? launch_gemm_wide(p, st) : p.M <= kTeamMaxRows ? launch_gemm_team(p, st) : launch_gemm_tc5(p, st);
+    if (e != cudaSuccess) return cuda_fail(e, launch_wide ? "w46_gemm_wide launch" : p.M <= kTeamMaxRows ? "w46_gemm_team launch" : "w46_gemm_tc5 launch");
   }
   return FP6M_OK;
 }

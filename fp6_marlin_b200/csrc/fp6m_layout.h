@@ -184,7 +184,15 @@ FP6M_HD long long range_cost(const Geometry& g, int u0, int u1) {
 
 // `row_tiles` > 1: the launch covers that many tiles of rows of A; the units of tile t follow those of
 // tile t - 1 (virtual strips), so a CTA mostly works on whole strips of one tile.
-inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_tiles = 1) {
+//
+// `reducer_penalty`: in the kernel for 33 to 128 rows a CTA whose range starts inside a strip and reaches the strip's end reduces
+// that strip at its own end: such CTAs get so many cost units (one segment) less work than the others - measured 1 to 2 % on
+// the steps of the Llama-2 layers; two or four segments less are no better.  (The kernel for more than 128 rows, which sums a
+// strip where it starts, gets the same shares when it has one tile of rows.  The kernels for up to 32 rows do that too and take 0:
+// measured no difference, and one round instead of four, which is most of the host time of a call.)
+// Which CTAs they are depends on the boundaries, so the shares are settled in a few rounds.
+constexpr int kReducerPenalty = 16;
+inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_tiles = 1, int reducer_penalty = kReducerPenalty) {
   if (ctas > kMaxCtas) ctas = kMaxCtas;
   if (ctas < 1) ctas = 1;
   const int ups = units_per_strip(g);
@@ -193,26 +201,29 @@ inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_ti
   const long long total_cost = (long long)row_tiles * ups * ((long long)kInt4UnitCost * g.strips4 + (long long)kFp6UnitCost * g.strips6);
   out->ctas = ctas;
   out->total_units = total_units;
-  // In the kernel for up to 128 rows a CTA whose range starts inside a strip and reaches the strip's end reduces that strip
-  // at its own end: such CTAs get `kReducerPenalty` cost units (one segment) less work than the others - measured 1 to 2 % on
-  // the steps of the Llama-2 layers; two or four segments less are no better.  (The kernel for more than 128 rows, which sums a
-  // strip where it starts, gets the same shares when it has one tile of rows.)
-  // Which CTAs they are depends on the boundaries, so the shares are settled in a few rounds.
-  constexpr int kReducerPenalty = 16;
+  const int rounds = (reducer_penalty > 0 && row_tiles == 1) ? 4 : 1;
+  const long long even = total_cost / ctas;         // equal targets without a 64-bit division per CTA: total_cost * c / ctas
+  const int rest = (int)(total_cost % ctas);
   double share[kMaxCtas];
-  for (int c = 0; c < ctas; ++c) share[c] = 1.0;
-  const int rounds = (kReducerPenalty > 0 && row_tiles == 1) ? 4 : 1;
+  if (rounds > 1)
+    for (int c = 0; c < ctas; ++c) share[c] = 1.0;
   for (int round = 0; round < rounds; ++round) {
     double share_total = 0.0;
-    for (int c = 0; c < ctas; ++c) share_total += share[c];
+    if (rounds > 1)
+      for (int c = 0; c < ctas; ++c) share_total += share[c];
     // bound[c] = first unit at which the cost of the units before it reaches CTA c's target, all of them in
     // one walk over the strips (the targets rise with c)
     int strip = 0, real = 0;          // the strip the walk is in; its index among the strips of one row tile
     long long acc = 0;                // cost of the units before that strip
     double before = 0.0;
     for (int c = 0; c < ctas; ++c) {
-      const long long target = rounds == 1 ? total_cost * c / ctas : (long long)((double)total_cost * (before / share_total));
-      before += share[c];
+      long long target;
+      if (rounds == 1) {
+        target = even * c + rest * c / ctas;
+      } else {
+        target = (long long)((double)total_cost * (before / share_total));
+        before += share[c];
+      }
       int cost = real < g.strips4 ? kInt4UnitCost : kFp6UnitCost;
       while (acc + (long long)ups * cost <= target) {
         acc += (long long)ups * cost;
@@ -220,7 +231,7 @@ inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_ti
         if (++real == nstrips) real = 0;
         cost = real < g.strips4 ? kInt4UnitCost : kFp6UnitCost;
       }
-      out->bound[c] = strip * ups + (int)((target - acc + cost - 1) / cost);
+      out->bound[c] = strip * ups + ((int)(target - acc) + cost - 1) / cost;       // less than a strip's cost: 32 bits
     }
     out->bound[ctas] = total_units;
     if (round + 1 < rounds) {
@@ -228,7 +239,7 @@ inline void make_schedule(const Geometry& g, int ctas, Schedule* out, int row_ti
       for (int c = 0; c < ctas; ++c) {
         const int u0 = out->bound[c], u1 = out->bound[c + 1];
         const bool reduces = (u0 % ups) != 0 && u1 >= (u0 / ups + 1) * ups;
-        share[c] = reduces ? 1.0 - (double)kReducerPenalty / per_cta : 1.0;
+        share[c] = reduces ? 1.0 - (double)reducer_penalty / per_cta : 1.0;
         if (share[c] < 0.25) share[c] = 0.25;
       }
     }

@@ -48,7 +48,7 @@ struct MulParams {
   int* status;          // optional device status word
   OutputMap out;
   int weights_early;    // the kernel before this one in the stream does not write B or S: read them before it has finished
-  int expand_early;     // (only with weights_early) kernel for up to 128 rows: the teams expand their first segments before the grid dependency
+  int expand_early;     // (only with weights_early) kernel for 33 to 128 rows: the teams expand their first segments before the grid dependency
   int vec_rows;         // kernel for more than 128 rows: finished rows leave as 16-byte stores (every row start and both
                         // column bases are multiples of 8 halves, no fused epilogue)
   int tile_rows;        // kernel for more than 128 rows: rows of a tile
@@ -73,6 +73,10 @@ bool tc5_get_overlap();
 void tc5_set_ordered_sums(bool on);
 bool tc5_get_ordered_sums();
 cudaError_t launch_gemm_tc5(const MulParams& p, cudaStream_t stream);
+
+// gemm_team.cu
+constexpr int kTeamMaxRows = 32;    // rows of A the kernel of gemm_team.cu covers
+cudaError_t launch_gemm_team(const MulParams& p, cudaStream_t stream);
 
 // gemm_wide.cu
 cudaError_t encode_activation_map(const half* A, int M, int K, int box_rows, CUtensorMap* map);

@@ -1,32 +1,29 @@
-// W(4&6)A16 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for up to 128 rows of A (instances for
-// 16, 32, 64 and 128 rows; the description below is that of the 16-row instance, the others differ in the
-// numbers of teams, stages and tiles - see the configurations at the end of the file).
+// W(4&6)A16 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for 33 to 128 rows of A (instances for 64 and 128
+// rows; fewer rows: gemm_team.cu and gemm_few.cu).
 //
 // The product is computed transposed, D[n, m] = sum_k W[k, n] * A[m, k]: the 128 weight columns of
 // a strip are the M dimension of tcgen05.mma (one TMEM lane per weight column), the rows of A are
-// its N dimension (16), and the dequantised weights are the A operand read from TENSOR MEMORY, so
-// they never travel through shared memory.  Legacy mma.sync costs about 32 cycles per m16n8k16
-// tile on B200 and cannot keep up with HBM; tcgen05 can: one 128 x 16 x 16 MMA occupies the tensor
-// pipe for about 32 cycles whatever its N, i.e. 256 cycles per 8 KB of INT4 weights.
+// its N dimension, and the dequantised weights are the A operand read from TENSOR MEMORY, so
+// they never travel through shared memory.
 //
 // Work unit: a SEGMENT = one 128-row block of one 128-column strip (two 64-row units, 8 KB of INT4
 // or 12 KB of FP6 words); the host hands every CTA a contiguous range of blocks in strip-major,
 // K-fastest order (fp6m_layout.h, boundaries on whole blocks).  One CTA per SM, five roles that
 // only meet at mbarriers:
 //   warp 0      weights producer: one bulk TMA copy (cp.async.bulk) per segment into a ring of
-//               shared-memory stages.  The first round of copies is issued by fifteen other warps, one
+//               shared-memory stages.  The first round of copies is issued by other warps, one
 //               stage each, before the rest of the CTA has finished its set-up.
-//   warp 1      activations producer: one tiled TMA copy per segment (2 units x 16 rows x 64 halves,
+//   warp 1      activations producer: one tiled TMA copy per segment (2 units x the rows x 64 halves,
 //               128-byte swizzle = the K-major swizzled B operand of the MMA; rows beyond M and
 //               units beyond K read as zero).
-//   warps 2-7   MMA issuers, two per dequantiser team (one per 64-row unit): four tcgen05.mma
+//   warps 2-5   MMA issuers, two per dequantiser team (one per 64-row unit): four tcgen05.mma
 //               (kind::f16, fp32 accumulators in TMEM) per segment each, all accumulating into a tile
-//               the team zeroed, then a commit (behind elect.sync, see elect_one: 11 to 15 cycles per MMA; behind `lane == 0`
-//               it was 175 beside busy teams, and K = N = 8192 at 16 / 64 rows took 13.8 / 20.8 us instead of 13.1 / 20.0).  The two
+//               that was zeroed, then a commit (behind elect.sync, see elect_one: 11 to 15 cycles per MMA; behind `lane == 0`
+//               it was 175 beside busy teams, and K = N = 8192 at 64 rows took 20.8 us instead of 20.0).  The two
 //               commits of a segment tell the epilogue warps that the accumulator tile is ready and
 //               the team and the activations producer that operand slot and activation tile are free.
-//               Warp 2 owns the TMEM allocation; warp 7 also reads the launch epoch.
-//   warps 8-19  three dequantiser TEAMS of four warps; thread = weight column = TMEM lane.  The teams
+//               Warp 2 owns the TMEM allocation; warp 5 also reads the launch epoch.
+//   warps 8-15  two dequantiser TEAMS of four warps; thread = weight column = TMEM lane.  The teams
 //               take the CTA's segments in turn.  A thread reads its 2 x 32 bytes of a segment,
 //               expands the sixteen words in registers and stores them with tcgen05.st into the
 //               segment's TMEM operand slot.  INT4 nibbles become the exact integers q - 8 in fp16
@@ -35,17 +32,14 @@
 //               FP6 codes become `s 00eee mm` fp16 patterns (exact value / 4096, as dequant_8fp6
 //               builds them before its multiply by 4096, :195-237).  A team never waits for an MMA of
 //               its own segment: it goes straight on to its next one.
-//   warps 20-27 epilogue: two sets of four warps (one warp per TMEM lane quarter); set e takes the
-//               segments n = e, e + 2, ...  Every segment has its own accumulator tile; an epilogue warp
-//               reads the tile back (tcgen05.ld), multiplies by the column's group scale in fp32 and
-//               adds to registers.  At the end of a slice (the CTA's blocks of one strip) set 1 hands its
-//               sums to set 0 through shared memory, and set 0 writes C (column scale in fp32, one
-//               rounding to fp16) or a split-K partial.  (One set alone needs ~700 cycles per segment:
-//               its chain wait - load - wait - add is serial.)
-// Rings: 15 weight stages, 6 {operand slot, activation tile, accumulator tile} entries.  Both ring sizes
+//   the others  epilogue: sets of four warps (one warp per TMEM lane quarter), each with its share of the rows.  An epilogue
+//               warp reads the tile of every segment back (tcgen05.ld), multiplies by the column's group scale in fp32 and
+//               adds to registers.  At the end of a slice (the CTA's blocks of one strip) it writes C (column scale in
+//               fp32, one rounding to fp16) or a split-K partial.
+// Rings: the sizes of the weight stages and of the {operand slot, activation tile, accumulator tile} entries
 // are multiples of the number of teams, so a stage or an entry always belongs to the same team and every
 // waiter of an mbarrier observes each of its phases in turn (a parity wait that skipped a phase would
-// pass early).  Instances whose tiles are too wide to have one per entry keep fewer tiles than entries: the
+// pass early).  The 128-row instance, whose tiles are too wide to have one per entry, keeps fewer tiles than entries: the
 // epilogue zeroes a tile after reading it and hands it to the issuers of the segment that uses it next.
 // The INT4 and the FP6 strips run through separate instantiations of the team loop, so that the
 // hot loop holds the instructions of one format only.
@@ -58,9 +52,8 @@
 // prefetch of its first round of weight copies run before griddepcontrol.wait, i.e. while the kernel before it
 // finishes.  With p.weights_early (the caller's switch: that kernel does not write this GEMM's weights) the copies
 // themselves are issued before the wait.  (Measured, eager back-to-back calls without the switch, against launches that
-// wait for their predecessor: K = N = 8192 at 16 rows 17.2 -> 14.2 us, the four GEMMs of a Llama-2-7B block at 5 rows
-// 67.4 -> 54.9, 4096 x 12288 at 48 rows 21.3 -> 18.7.)  Every role passes the wait before its first bounded wait, so a
-// long-running predecessor cannot run the bounds out.
+// wait for their predecessor: 4096 x 12288 at 48 rows 21.3 -> 18.7 us.)  Every role passes the wait before its first bounded
+// wait, so a long-running predecessor cannot run the bounds out.
 //
 // Replaces the reference's fp6_kernel_marlin (fp6_marlin/fp6_marlin_cuda_kernel.cu:288-837).
 #include <cuda_fp16.h>
@@ -101,8 +94,7 @@ struct Tc5Cfg {
   // eight warps in front of them (producers, issuers, two spare warps), sixteen rows each.
   // (measured at 128 rows, K = N = 8192: 32.0 -> 27.7 us per GEMM; K = N = 4096: 26.0 -> 19.9.  Unequal shares -
   // fewer rows for the epilogue sets, which get there last - measured: 128 rows, sets x 8 + the others x 24: 30.0 us;
-  // 64 rows, sets x 8 + teams and front warps x 12: the same as four groups; 32 rows, sets x 4 + three teams x 8:
-  // -1.7 %, but the 16-row instance compiled from that source ran 0.7 % slower.)
+  // 64 rows, sets x 8 + teams and front warps x 12: the same as four groups.)
   static constexpr int kReduceGroups = (kEpiSets == 4 && kTeams == 2 && kDeqBase == 8) ? 8 : 4;
   static_assert(kTeams >= 2 && STAGES_ <= 4 * kTeams + 4 * kEpiSets, "the first round of weight copies is issued by one warp per stage");
   static constexpr int kEpochWarp = 2 + kIssuers - 1;
@@ -115,7 +107,7 @@ struct Tc5Cfg {
   static constexpr int kDRing = DRING_;
   static constexpr bool kDecoupled = kDRing != kRing;
   static_assert(kDRing <= kRing && kDRing % 2 == 0, "accumulator tiles");
-  static_assert(!kDecoupled || NT_ > 16, "with fewer tiles than entries both epilogue sets read every segment");
+  static_assert(NT_ > 16, "every epilogue set reads its share of the rows of every segment");
   static constexpr int kActUnitBytes = NT * 128;       // NT rows x 64 halves
   static constexpr int kActBytes = 2 * kActUnitBytes;
   static constexpr int kNumBars = 2 * kStages + 4 * kRing + 1;
@@ -128,13 +120,8 @@ struct Tc5Cfg {
   // the group scale (fp16 bits in a word) of every column of the segment in a ring entry; with fewer
   // accumulator tiles than entries a team may be a whole round ahead of the epilogue: two sets of scales
   static constexpr int kScaleRingBytes = (kDecoupled ? 2 : 1) * kRing * kStripCols * 4;
-  // Up to 16 rows the two epilogue sets take the segments in turn and pool their sums at the end of a slice;
-  // with more rows each set reads its half of the rows of every segment (the sums would not fit in registers).
-  static constexpr bool kRowSplit = NT > 16;
-  static constexpr int kEpiRows = kRowSplit ? NT / kEpiSets : NT;     // rows a thread of an epilogue set accumulates
-  static constexpr int kXchBytes = kRowSplit ? 0 : NT * kStripCols * 4;   // the second epilogue set's sums of a slice
-  static_assert(kRowSplit || kRing % kEpiSets == 0, "a ring entry always belongs to the same epilogue set");
-  static constexpr int kSmemBytes = kStages * kStageW + kRing * kActBytes + kScaleRingBytes + kXchBytes + kNumBars * 8 + 64 + 1024;   // + alignment slack
+  static constexpr int kEpiRows = NT / kEpiSets;       // rows a thread of an epilogue set accumulates
+  static constexpr int kSmemBytes = kStages * kStageW + kRing * kActBytes + kScaleRingBytes + kNumBars * 8 + 64 + 1024;   // + alignment slack
   static constexpr int kTmemD = 0, kTmemA = kDRing * NT;  // accumulator tiles, then operand slots of 64 columns
   static constexpr int kTmemUsed = kTmemA + kRing * 64;
   static constexpr int kTmemCols = kTmemUsed <= 128 ? 128 : (kTmemUsed <= 256 ? 256 : 512);
@@ -142,78 +129,6 @@ struct Tc5Cfg {
   static constexpr int kSlotFloats = NT * kStripCols;
   static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 };
-
-// activations of one segment: the box {64 halves, NT rows, 2 units} at unit `unit` of K
-__device__ __forceinline__ void tma_load_act_segment(uint32_t dst, const CUtensorMap* map, int unit, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-               ::"r"(dst), "l"(map), "r"(0), "r"(0), "r"(unit), "r"(bar) : "memory");
-}
-
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-  return v;
-}
-
-// Bytes of one segment of (linear) strip `s`.
-__device__ __forceinline__ uint32_t segment_bytes(const Geometry& geo, int s) {
-  return s < geo.strips4 ? 2u * strip_quads(geo.n4, s) * kInt4UnitQuadBytes
-                         : 2u * strip_quads(geo.n6, s - geo.strips4) * kFp6UnitQuadBytes;
-}
-// Byte offset of block `blk` of strip `s` in the packed weights (blocks of a strip, and strips, follow
-// one another without gaps).
-__device__ __forceinline__ int64_t segment_offset(const Geometry& geo, int s, int blk) {
-  return s < geo.strips4 ? int4_unit_offset(geo, s, 2 * blk) : fp6_unit_offset(geo, s - geo.strips4, 2 * blk);
-}
-
-// Group scales of one segment: nq * 64 bytes behind the packed words of its stage (FP6 and per-channel strips
-// have none).  Offset of the scales inside a stage: INT4 segments fill at most 8192 of the kStageW bytes.
-constexpr uint32_t kStageScaleOff = 8192;
-__device__ __forceinline__ uint32_t segment_scale_bytes(const Geometry& geo, int s) {
-  return (s < geo.strips4 && geo.groups > 1) ? (uint32_t)strip_quads(geo.n4, s) * kQuadCols * 2u : 0u;
-}
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void sts_f32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
-__device__ __forceinline__ void sts_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
-  unsigned short v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return v;
-}
-
-// Expands one 64-row unit of this thread's column (eight packed words, plus four two-bit words for FP6)
-// into 32 TMEM columns at a_tmem.
-template <bool IS6>
-__device__ __forceinline__ void expand_words(const uint4& lo, const uint4& hi, const uint4& two, uint32_t a_tmem) {
-  const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-  if constexpr (IS6) {
-    const uint32_t twos[4] = {two.x, two.y, two.z, two.w};
-#pragma unroll
-    for (int step = 0; step < 4; ++step) {
-      uint32_t regs[8];
-      expand_fp6(words[2 * step], twos[step], 0, regs);
-      expand_fp6(words[2 * step + 1], twos[step], 4, regs + 4);
-      tc_st8(a_tmem + step * 8, regs);
-    }
-  } else {
-#pragma unroll
-    for (int step = 0; step < 4; ++step) {
-      uint32_t regs[8];
-      expand_int4(words[2 * step], regs);
-      expand_int4(words[2 * step + 1], regs + 4);
-      tc_st8(a_tmem + step * 8, regs);
-    }
-  }
-}
 
 template <class C>
 __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __grid_constant__ MulParams p, const __grid_constant__ CUtensorMap amap) {
@@ -223,8 +138,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t act_base = smem0 + S * kStageW;
   const uint32_t scale_ring = act_base + R * C::kActBytes;      // [entry][column] fp32
-  const uint32_t xch = scale_ring + C::kScaleRingBytes;         // [row][column] fp32
-  const uint32_t bars0 = xch + C::kXchBytes;
+  const uint32_t bars0 = scale_ring + C::kScaleRingBytes;
   const uint32_t w_full = bars0, w_empty = w_full + 8 * S;
   const uint32_t act_full = w_empty + 8 * S, ready = act_full + 8 * R, done = ready + 8 * R;
   const uint32_t d_free = done + 8 * R;        // the accumulator tile has been read back
@@ -292,7 +206,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
     // act_full: expect_tx arrival of the activations producer; ready: every thread of the segment's team
     // stored its operands into TMEM; done: the commit(s) of the segment's issuer(s); d_free: every thread of
     // the entry's epilogue set has read the tile.  (All lanes arrive: no election, no branch.)
-    const uint32_t count = i < R ? 1u : (i < 2 * R ? 128u : (i < 3 * R ? (C::kSplitIssue ? 2u : 1u) : (i < 4 * R ? (C::kRowSplit ? 128u * C::kEpiSets : 128u) : 1u)));
+    const uint32_t count = i < R ? 1u : (i < 2 * R ? 128u : (i < 3 * R ? (C::kSplitIssue ? 2u : 1u) : (i < 4 * R ? 128u * C::kEpiSets : 1u)));
     mbar_init(act_full + 8 * i, count);
     mbar_fence_init();
   }
@@ -671,15 +585,13 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
     else if (C::kEpiSets == 2 && team < 2) reduce_shared_strip(2 + team);
   } else if (warp >= C::kEpiBase) {
     // ================================================================== epilogue
-    // Two sets of one warp per lane quarter; thread = weight column.  Set e reads the accumulator tiles of
-    // the segments n = e, e + 2, ... back, scales and accumulates; at the end of a slice set 1 passes its
-    // sums to set 0, which writes the slice out (sums added in the order set 0 + set 1: fixed).
-    constexpr int kEpiThreads = 128 * C::kEpiSets;
+    // Sets of one warp per lane quarter; thread = weight column.  Every set reads its rows of the accumulator tile of
+    // every segment back, scales and accumulates, and writes them out at the end of a slice.
     const int eset = (warp - C::kEpiBase) >> 2;
     const uint32_t d_base = tmem + ((uint32_t)(quarter * 32) << 16) + C::kTmemD;       // + r * NT
 
     constexpr int ROWS = C::kEpiRows;
-    const int row0 = C::kRowSplit ? eset * ROWS : 0;          // this set's rows of A and C (all of them when the sets take turns)
+    const int row0 = eset * ROWS;          // this set's rows of A and C
     auto write_strip = [&](const Slice& sl, const float (&v)[ROWS]) {
       const int ncols = strip_cols(sl.is6 ? geo.n6 : geo.n4, sl.strip);
       const bool writes = c < ncols;
@@ -704,9 +616,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
     float acc[ROWS];
 #pragma unroll
     for (int m = 0; m < ROWS; ++m) acc[m] = 0.f;
-    constexpr int kStep = C::kRowSplit ? 1 : C::kEpiSets;      // segments from one of this set's to its next
-    if (!C::kRowSplit && eset == 0) named_bar_arrive(2, kEpiThreads);       // the exchange buffer starts out free
-    int n = C::kRowSplit ? 0 : eset, r = n, n_first = 0;    // n_first: first segment of the current slice
+    int n = 0, r = 0, n_first = 0;                 // n_first: first segment of the current slice
     uint32_t rphase = 0;
     if constexpr (C::kDecoupled) {
       // the accumulator tiles start out free; when two issuers add to a tile it must start out zero
@@ -724,7 +634,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
       const int n_end = min(nseg, (s + 1) * kb - B0);
       const Slice sl = open_slice(s, b0, b0 + (n_end - n_first));
 #pragma unroll 1
-      for (; n < n_end; n += kStep) {
+      for (; n < n_end; ++n) {
         float scale;
         uint32_t d_tile;
         if constexpr (C::kDecoupled) {
@@ -762,26 +672,11 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
           mbar_arrive(d_free + 8 * r);                  // the team may zero the tile for its next segment
         }
         FP6M_TRACE_EVENT(trace, 16, n);
-        r += kStep;
-        if (r >= R) { r -= R; rphase ^= 1; }
+        if (++r == R) { r = 0; rphase ^= 1; }
       }
       n_first = n_end;
       FP6M_TRACE_EVENT(trace, 20, s);
-      if constexpr (C::kRowSplit) {
-        finish_slice(sl, acc);
-      } else if (eset == 1) {
-        // set 0 has read the previous slice's sums out of the exchange buffer (barrier 2); publish (barrier 1)
-        named_bar_sync(2, kEpiThreads);
-#pragma unroll
-        for (int m = 0; m < ROWS; ++m) sts_f32(xch + (m * kStripCols + c) * 4, acc[m]);
-        named_bar_arrive(1, kEpiThreads);
-      } else {
-        named_bar_sync(1, kEpiThreads);
-#pragma unroll
-        for (int m = 0; m < ROWS; ++m) acc[m] += lds_f32(xch + (m * kStripCols + c) * 4);
-        named_bar_arrive(2, kEpiThreads);
-        finish_slice(sl, acc);
-      }
+      finish_slice(sl, acc);
       FP6M_TRACE_EVENT(trace, 22, s);
 #pragma unroll
       for (int m = 0; m < ROWS; ++m) acc[m] = 0.f;
@@ -812,20 +707,10 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_tc5_kernel(const __gr
   }
 }
 
-#ifndef FP6M_TC5_TEAMS
-#define FP6M_TC5_TEAMS 3
-#define FP6M_TC5_STAGES 15
-#endif
-using Tc5Rows16 = Tc5Cfg<16, FP6M_TC5_STAGES, 2 * FP6M_TC5_TEAMS, FP6M_TC5_TEAMS, true>;          // 3 teams: 6 x 16 + 6 x 64 = 480 TMEM columns
-using Tc5Rows16Ordered = Tc5Cfg<16, FP6M_TC5_STAGES, 2 * FP6M_TC5_TEAMS, FP6M_TC5_TEAMS, false>;  // one issuing thread per accumulator tile: run-to-run bit-identical
-// 17 to 32 rows: three teams and six operand slots as above, four accumulator tiles of 32 TMEM columns.
 // 33 to 64 rows: two teams, four operand slots and four accumulator tiles of 64 columns (with six slots only two
 // tiles fit, and the chain MMA -> read-back -> next MMA on two tiles is as slow as two teams).
-// The activation tiles grow with the rows, the weight stages give way.
-using Tc5Rows32 = Tc5Cfg<32, 12, 6, 3, true, 4>;
-using Tc5Rows32Ordered = Tc5Cfg<32, 12, 6, 3, false, 4>;
 using Tc5Rows64 = Tc5Cfg<64, 10, 4, 2, true>;
-using Tc5Rows64Ordered = Tc5Cfg<64, 10, 4, 2, false>;
+using Tc5Rows64Ordered = Tc5Cfg<64, 10, 4, 2, false>;          // one issuing thread per accumulator tile: run-to-run bit-identical
 
 // 65 to 128 rows: two teams, four operand slots (256 TMEM columns) beside two accumulator tiles of 128 columns;
 // four epilogue sets of 32 rows each
@@ -894,8 +779,6 @@ size_t tc5_scratch_bytes(int ctas, int rows) {
 // Runs the GEMM for rows [0, p.M) with p.M <= kTc5MaxRows.  The schedule's unit boundaries must be even (whole blocks).
 cudaError_t launch_gemm_tc5(const MulParams& p, cudaStream_t stream) {
   switch (tc5_tile_rows(p.M)) {
-    case 16: return g_ordered_sums ? launch_tc5<Tc5Rows16Ordered>(p, stream) : launch_tc5<Tc5Rows16>(p, stream);
-    case 32: return g_ordered_sums ? launch_tc5<Tc5Rows32Ordered>(p, stream) : launch_tc5<Tc5Rows32>(p, stream);
     case 64: return g_ordered_sums ? launch_tc5<Tc5Rows64Ordered>(p, stream) : launch_tc5<Tc5Rows64>(p, stream);
     default: return g_ordered_sums ? launch_tc5<Tc5Rows128Ordered>(p, stream) : launch_tc5<Tc5Rows128>(p, stream);
   }

@@ -146,7 +146,7 @@ __device__ __forceinline__ void store_column_rows(const Params& p, int row0, boo
     }
     return;
   }
-  if (kRows % 4 == 0 && kRows >= 8 && p.vec_rows) {
+  if constexpr (kRows % 4 == 0 && kRows >= 8) if (p.vec_rows) {
     // Four neighbouring lanes turn their 4 x kRows block round with shuffles: lane q of the quad ends up
     // with the rows q * kRows / 4 ... of all four columns and stores 8 bytes per row instead of 2 (a warp
     // store then covers four rows of 64 bytes; the host checked that every row start and both column
@@ -275,6 +275,143 @@ __device__ __forceinline__ void expand_fp6_scaled(uint32_t four, uint32_t two, i
   expand_fp6(four, two, rot, e);
 #pragma unroll
   for (int i = 0; i < 4; ++i) b[i] = h2_as_u32(__hmul2(u32_as_h2(e[i]), s4096));
+}
+
+// ---- segments (one 128-row block of one strip) in shared memory ------------------------------------------------
+// activations of one segment: the box {64 halves, NT rows, 2 units} at unit `unit` of K
+__device__ __forceinline__ void tma_load_act_segment(uint32_t dst, const CUtensorMap* map, int unit, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(dst), "l"(map), "r"(0), "r"(0), "r"(unit), "r"(bar) : "memory");
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+
+// Bytes of one segment of (linear) strip `s`.
+__device__ __forceinline__ uint32_t segment_bytes(const Geometry& geo, int s) {
+  return s < geo.strips4 ? 2u * strip_quads(geo.n4, s) * kInt4UnitQuadBytes
+                         : 2u * strip_quads(geo.n6, s - geo.strips4) * kFp6UnitQuadBytes;
+}
+// Byte offset of block `blk` of strip `s` in the packed weights (blocks of a strip, and strips, follow
+// one another without gaps).
+__device__ __forceinline__ int64_t segment_offset(const Geometry& geo, int s, int blk) {
+  return s < geo.strips4 ? int4_unit_offset(geo, s, 2 * blk) : fp6_unit_offset(geo, s - geo.strips4, 2 * blk);
+}
+
+// Group scales of one segment: nq * 64 bytes behind the packed words of its stage (FP6 and per-channel strips
+// have none).  Offset of the scales inside a stage: INT4 segments fill at most 8192 of the kStageW bytes.
+constexpr uint32_t kStageScaleOff = 8192;
+__device__ __forceinline__ uint32_t segment_scale_bytes(const Geometry& geo, int s) {
+  return (s < geo.strips4 && geo.groups > 1) ? (uint32_t)strip_quads(geo.n4, s) * kQuadCols * 2u : 0u;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float lds_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_f32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return v;
+}
+
+// Expands one 64-row unit of this thread's column (eight packed words, plus four two-bit words for FP6)
+// into 32 TMEM columns at a_tmem.
+template <bool IS6>
+__device__ __forceinline__ void expand_words(const uint4& lo, const uint4& hi, const uint4& two, uint32_t a_tmem) {
+  const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  if constexpr (IS6) {
+    const uint32_t twos[4] = {two.x, two.y, two.z, two.w};
+#pragma unroll
+    for (int step = 0; step < 4; ++step) {
+      uint32_t regs[8];
+      expand_fp6(words[2 * step], twos[step], 0, regs);
+      expand_fp6(words[2 * step + 1], twos[step], 4, regs + 4);
+      tc_st8(a_tmem + step * 8, regs);
+    }
+  } else {
+#pragma unroll
+    for (int step = 0; step < 4; ++step) {
+      uint32_t regs[8];
+      expand_int4(words[2 * step], regs);
+      expand_int4(words[2 * step + 1], regs + 4);
+      tc_st8(a_tmem + step * 8, regs);
+    }
+  }
+}
+
+
+// ---- strips shared by several CTAs, kernels for up to 32 rows -------------------------------------------------
+// Partials are {value, tag} words as in the other kernels; the CTA in which a strip STARTS sums it.  That slice is the CTA's
+// last one, while the others left theirs at the start of their ranges (a CTA has one partial: only its first slice can
+// start inside a strip).  The kernels hand the ranges out from the last to the first, so a CTA only waits for CTAs that
+// were dispatched before it.
+// `rows` is the height of a slot, `row0` the first of this thread's RR rows, `c` its column.
+template <int RR, class Params>
+__device__ __forceinline__ void store_partial(const Params& p, int cta, int rows, int row0, int c, uint32_t tag, const float (&out)[RR]) {
+  unsigned long long* slot = p.partials + ((size_t)cta * rows + row0) * kStripCols + c;
+#pragma unroll
+  for (int m = 0; m < RR; ++m) st_relaxed_u64(slot + m * kStripCols, ((unsigned long long)tag << 32) | __float_as_uint(out[m]));
+}
+// adds the partials of the CTAs behind `cta` whose ranges start before block `s_end`, in the order of the ranges; up to sixteen
+// tagged words in flight per thread
+template <int RR, class Params>
+__device__ __forceinline__ void add_partials(const Params& p, int cta, int s_end, int rows, int row0, int c, uint32_t tag, float (&out)[RR], WaitState& ws) {
+  constexpr int kBatch = RR < 16 ? 16 / RR : 1;
+#pragma unroll 1
+  for (int cc = cta + 1; cc < (int)gridDim.x && (p.sched.bound[cc] >> 1) < s_end; cc += kBatch) {
+    bool live[kBatch];
+    const unsigned long long* src[kBatch];
+    unsigned long long v[kBatch][RR];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int ci = cc + i;
+      live[i] = ci < (int)gridDim.x && (p.sched.bound[ci] >> 1) < s_end && p.sched.bound[ci] < p.sched.bound[ci + 1];     // a CTA without work stored nothing
+      src[i] = p.partials + ((size_t)(live[i] ? ci : cc) * rows + row0) * kStripCols + c;
+    }
+    bool all_here = false;
+#pragma unroll 1
+    for (int spin = 0; spin < (1 << 20) && !all_here; ++spin) {
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i)
+#pragma unroll
+        for (int m = 0; m < RR; ++m) v[i][m] = live[i] ? ld_relaxed_u64(src[i] + m * kStripCols) : 0;
+      all_here = true;
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i)
+#pragma unroll
+        for (int m = 0; m < RR; ++m) all_here = all_here && (!live[i] || (uint32_t)(v[i][m] >> 32) == tag);
+      if (ws.failed) break;                       // a wait of this thread ran out before: do not wait again
+    }
+    if (!all_here) ws.failed = 1;
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i)
+#pragma unroll
+      for (int m = 0; m < RR; ++m) out[m] += live[i] ? __uint_as_float((uint32_t)v[i][m]) : 0.f;
+  }
+  __syncwarp();
+}
+// column scale: per-channel INT4: s; FP6: s * 4096; group INT4: already applied
+template <class Params>
+__device__ __forceinline__ float strip_column_scale(const Params& p, bool is6, int strip, int c, bool writes) {
+  if (!writes || (!is6 && p.geo.groups > 1)) return 1.f;
+  const half* sp = p.S + (is6 ? fp6_scale_offset(p.geo, strip) : int4_scale_offset(p.geo, strip, 0));
+  return __half2float(__ldg(sp + c)) * (is6 ? 4096.f : 1.f);
 }
 
 }  // namespace fp6m

@@ -1,10 +1,10 @@
-"""In-kernel timeline of the GEMM for up to 128 rows (developer tool; needs a B200).
+"""In-kernel timeline of the GEMM for 33 to 128 rows (developer tool; needs a B200).
 
 The library built with ``python fp6_marlin_b200/build.py --trace`` records, in two CTAs of every launch,
 {tag, argument, SM clock} events of every warp (csrc/trace.cuh), and the start and end of every CTA of the
 last 64 launches in nanoseconds.  This module runs a few launches and prints both:
 
-    FP6M_LIB=fp6_marlin_b200/libfp6m_trace.so python -m fp6_marlin_b200.timeline 8192,8192,16
+    FP6M_LIB=fp6_marlin_b200/libfp6m_trace.so python -m fp6_marlin_b200.timeline 8192,8192,64
 
 ``timeline``  per segment n of a traced CTA, in SM cycles since the CTA started: when its dequantiser team
               began it, found its ring entry free, had expanded it, had loaded the next segment's words, saw
@@ -58,7 +58,7 @@ def timeline(k, n, m):
     buf = np.zeros((CTAS_TRACED, WARPS, ENTRIES), dtype=np.uint64)
     rc = read(buf.ctypes.data, buf.nbytes)
     print("trace_read rc", rc, "device status", fm.device_status(dev))
-    teams = 3 if m <= 32 else 2          # dequantiser teams of the kernel instance for m rows
+    teams = 2                            # dequantiser teams of the kernel
     deq = (2 + 2 * teams + 3) & ~3
     epi = deq + 4 * teams
     for ci in range(CTAS_TRACED):
@@ -148,8 +148,10 @@ def launches(k, n, m):
 
 
 if __name__ == "__main__":
-    shape = tuple(int(x) for x in (sys.argv[1] if len(sys.argv) > 1 else "8192,8192,16").split(","))
+    shape = tuple(int(x) for x in (sys.argv[1] if len(sys.argv) > 1 else "8192,8192,64").split(","))
     mode = sys.argv[2] if len(sys.argv) > 2 else "both"
+    if not 32 < shape[2] <= 128:
+        raise SystemExit("the timeline is built into the kernel for 33 to 128 rows")
     if mode in ("timeline", "both"):
         timeline(*shape)
     if mode in ("launches", "both"):

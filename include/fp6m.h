@@ -232,11 +232,11 @@ int fp6m_gather_columns(const void* c, void* y, const void* src, const void* bia
 int fp6m_set_launch_overlap(int enable);
 
 /* Process-wide option, off by default; returns the previous setting (a negative argument only queries).
- * The GEMM for up to 128 rows of A normally lets two threads issue the tensor-core instructions of one
+ * The GEMM for 33 to 128 rows of A normally lets two threads issue the tensor-core instructions of one
  * 128-row block, one per 64-row half, into one accumulator: the hardware may retire the halves in either
  * order, so the last bit of a result can differ between two runs on the same inputs (same products, same
  * fp32 adds, different order).  When on, one thread issues a block's instructions in a fixed order and two
- * runs agree bit for bit, at some cost in speed.  The reference's serial, lock-ordered reduction is
+ * runs agree bit for bit, at some cost in speed (GEMMs of fewer or more rows always do).  The reference's serial, lock-ordered reduction is
  * deterministic (fp6_marlin_cuda_kernel.cu:645-696). */
 int fp6m_set_ordered_sums(int enable);
 

@@ -225,8 +225,10 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     make_schedule(p.geo, launch_ctas, &p.sched, p.row_tiles, !launch_wide && p.M <= kTeamMaxRows ? 0 : kReducerPenalty);
     align_schedule_to_blocks(&p.sched);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t e = launch_wide ? launch_gemm_wide(p, st) : p.M <= kTeamMaxRows ? launch_gemm_team(p, st) : launch_gemm_tc5(p, st);
-    if (e != cudaSuccess) return cuda_fail(e, launch_wide ? "w46_gemm_wide launch" : p.M <= kTeamMaxRows ? "w46_gemm_team launch" : "w46_gemm_tc5 launch");
+    // the lines between the kernels: measured at 5, 8, 16 and 32 rows, see the heads of gemm_few.cu and gemm_team.cu
+    cudaError_t e = launch_wide ? launch_gemm_wide(p, st)
+                    : p.M <= kFewMaxRows ? launch_gemm_few(p, st) : p.M <= kTeamMaxRows ? launch_gemm_team(p, st) : launch_gemm_tc5(p, st);
+    if (e != cudaSuccess) return cuda_fail(e, launch_wide ? "w46_gemm_wide launch" : p.M <= kFewMaxRows ? "w46_gemm_few launch" : p.M <= kTeamMaxRows ? "w46_gemm_team launch" : "w46_gemm_tc5 launch");
   }
   return FP6M_OK;
 }

@@ -74,6 +74,10 @@ void tc5_set_ordered_sums(bool on);
 bool tc5_get_ordered_sums();
 cudaError_t launch_gemm_tc5(const MulParams& p, cudaStream_t stream);
 
+// gemm_few.cu
+constexpr int kFewMaxRows = 8;      // rows of A the kernel of gemm_few.cu covers
+cudaError_t launch_gemm_few(const MulParams& p, cudaStream_t stream);
+
 // gemm_team.cu
 constexpr int kTeamMaxRows = 32;    // rows of A the kernel of gemm_team.cu covers
 cudaError_t launch_gemm_team(const MulParams& p, cudaStream_t stream);

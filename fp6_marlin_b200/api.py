@@ -12,6 +12,7 @@ PyTorch is used for memory, streams and device management only.
 """
 from __future__ import annotations
 
+import ctypes
 import weakref
 
 import torch
@@ -19,6 +20,13 @@ from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import lib
+
+try:
+    from . import _call
+except ImportError as e:
+    raise ImportError(f"fp6_marlin_b200/_call.so is missing or does not load ({e}): build it with `python fp6_marlin_b200/build.py`") from e
+
+_call.bind(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in ("fp6m_mul", "fp6m_mul_fused", "fp6m_mul_scratch_bytes")))
 
 
 def _ptr(t: torch.Tensor) -> int:
@@ -307,6 +315,7 @@ def _device_buffers(device: torch.device, shape=None, stream=None):
     if idx not in _status:
         _status[idx] = torch.zeros(1, dtype=torch.int32, device=device)
         _sm_count[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
+        _call.set_device(idx, _ptr(_status[idx]), _sm_count[idx])
     need_key = (idx, shape)
     nbytes = _scratch_need.get(need_key)
     if nbytes is None:
@@ -324,6 +333,7 @@ def _device_buffers(device: torch.device, shape=None, stream=None):
         with torch.cuda.device(device):
             buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
         _scratch[key] = buf
+        _call.set_scratch(idx, key[1], _ptr(buf), nbytes)
     return idx, buf, _status[idx]
 
 
@@ -337,9 +347,10 @@ def set_launch_overlap(enable: bool) -> bool:
 
 
 def set_ordered_sums(enable: bool) -> bool:
-    """Process-wide switch (off by default); returns the previous setting.  When on, the GEMM for up to 16
+    """Process-wide switch (off by default); returns the previous setting.  When on, the GEMM for 33 to 128
     rows adds the products of a 128-row block in one fixed order, so two runs on the same inputs agree bit
-    for bit; when off, the two 64-row halves of a block may be added in either order (faster)."""
+    for bit; when off, the two 64-row halves of a block may be added in either order (faster).  GEMMs of fewer or more rows
+    always add in one order."""
     return bool(lib.fp6m_set_ordered_sums(1 if enable else 0))
 
 
@@ -357,15 +368,23 @@ def device_status(device=None) -> int:
     return value
 
 
-def _prepared_from_reference(B, s, k, n, quant_cols):
-    """Reference-layout tensors are re-tiled once and remembered for as long as `B` lives and is
-    not modified in place."""
-    key = id(B)
-    hit = _prepared.get(key)
+def _prepared_before(B, s, k, n, quant_cols):
+    """What :func:`_prepared_from_reference` remembers for these tensors, or None."""
+    hit = _prepared.get(id(B))
     if hit is not None:
         ref, ver, s_ref, s_ver, shape, packed = hit
         if ref() is B and ver == B._version and s_ref() is s and s_ver == s._version and shape == (k, n, quant_cols):
             return packed
+    return None
+
+
+def _prepared_from_reference(B, s, k, n, quant_cols):
+    """Reference-layout tensors are re-tiled once and remembered for as long as `B` lives and is
+    not modified in place."""
+    packed = _prepared_before(B, s, k, n, quant_cols)
+    if packed is not None:
+        return packed
+    key = id(B)
     packed = repack_from_reference(B, s, k, n, quant_cols)
     _prepared[key] = (weakref.ref(B, lambda _r, key=key: _prepared.pop(key, None)), B._version,
                       weakref.ref(s), s._version, (k, n, quant_cols), packed)
@@ -385,6 +404,21 @@ def mul(A, B, C, s, workspace, quant_cols=-1, thread_k=-1, thread_n=-1, sms=-1, 
     order.  Raises ``RuntimeError`` for the cases the reference raises for: workspace too small,
     ``N % thread_n`` or ``K % thread_k`` non-zero, no kernel for the tile shape.
     """
+    # plain CUDA tensors that pass every check: one call into native code; anything else takes the general path below
+    if layout == "b200":
+        rc = _call.mul(A, B, C, s, workspace, quant_cols, thread_k, thread_n, sms, max_par, group_size, _lib.EPILOGUE_NONE, None)
+        if rc == _lib.OK:
+            return
+        if rc > 0:
+            _raise_mul(rc, A.shape[0], C.shape[1], A.shape[1], thread_k, thread_n, max_par)
+    elif layout == "reference" and id(B) in _prepared and group_size <= 0 and A.dim() == 2 and C.dim() == 2 and B.is_contiguous() and s.is_contiguous():
+        packed = _prepared_before(B, s, A.shape[1], C.shape[1], quant_cols)
+        if packed is not None:
+            rc = _call.mul(A, packed[0], C, packed[1], workspace, quant_cols, thread_k, thread_n, sms, max_par, -1, _lib.EPILOGUE_NONE, None)
+            if rc == _lib.OK:
+                return
+            if rc > 0:
+                _raise_mul(rc, A.shape[0], C.shape[1], A.shape[1], thread_k, thread_n, max_par)
     if not A.is_cuda:
         raise RuntimeError("fp6_marlin_b200.mul needs CUDA tensors: there is no CPU implementation")
     M, K = A.shape[0], A.shape[1]
@@ -422,8 +456,12 @@ def mul(A, B, C, s, workspace, quant_cols=-1, thread_k=-1, thread_n=-1, sms=-1, 
                       _ptr(workspace), workspace.numel() * workspace.element_size(),
                       _ptr(scratch), scratch.numel(), dev_index, stream,
                       thread_k, thread_n, sms, max_par, quant_cols, group_size, _lib.LAYOUT_B200, _ptr(status))
-    if rc == _lib.OK:
-        return
+    if rc != _lib.OK:
+        _raise_mul(rc, M, N, K, thread_k, thread_n, max_par)
+
+
+def _raise_mul(rc, M, N, K, thread_k, thread_n, max_par):
+    """The exception for a status of fp6m_mul."""
     if rc == _lib.ERR_PROB_SHAPE:
         raise RuntimeError(f"Problem (m={M}, n={N}, k={K}) not compatible with thread_k={thread_k}, thread_n={thread_n}.")
     if rc == _lib.ERR_KERN_SHAPE:
@@ -452,6 +490,11 @@ def mul_fused(A, B, C, s, workspace, quant_cols=-1, *, epilogue="none", residual
     code = {"none": _lib.EPILOGUE_NONE, "silu_mul": _lib.EPILOGUE_SILU_MUL, "residual": _lib.EPILOGUE_RESIDUAL}.get(epilogue)
     if code is None:
         raise ValueError(f"mul_fused: unknown epilogue {epilogue!r}")
+    rc = _call.mul(A, B, C, s, workspace, quant_cols, -1, -1, sms, max_par, group_size, code, residual)
+    if rc == _lib.OK:
+        return
+    if rc > 0:
+        _raise_mul_fused(rc)
     if not A.is_cuda:
         raise RuntimeError("fp6_marlin_b200.mul_fused needs CUDA tensors: there is no CPU implementation")
     M, K = A.shape
@@ -478,10 +521,14 @@ def mul_fused(A, B, C, s, workspace, quant_cols=-1, *, epilogue="none", residual
                             _ptr(workspace), workspace.numel() * workspace.element_size(),
                             _ptr(scratch), scratch.numel(), dev_index, stream,
                             -1, -1, sms, max_par, quant_cols, group_size, _lib.LAYOUT_B200, _ptr(status), code, res_ptr)
+    if rc:
+        _raise_mul_fused(rc)
+
+
+def _raise_mul_fused(rc):
     if rc == _lib.ERR_CUDA:
         raise RuntimeError(f"fp6m_mul_fused: CUDA error: {_lib.last_cuda_error()}")
-    if rc:
-        raise RuntimeError(f"fp6m_mul_fused failed with code {rc}")
+    raise RuntimeError(f"fp6m_mul_fused failed with code {rc}")
 
 
 _PLAIN_TENSORS = (torch.Tensor, torch.nn.Parameter)

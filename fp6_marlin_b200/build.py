@@ -5,14 +5,18 @@ work before the package itself can be imported)
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libfp6m.so")
+CALL_PATH = os.path.join(PKG_DIR, "_call.so")          # extension module: the Python call path of mul and mul_fused
+CALL_SOURCE = "py_call.cpp"
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 
 CUDA_SOURCES = ["c_api.cu", "gemm_few.cu", "gemm_team.cu", "gemm_tc5.cu", "gemm_wide.cu", "dump_operands.cu", "prep_gpu.cu", "gather_columns.cu", "peer.cu"]
@@ -43,10 +47,28 @@ def needs_build() -> bool:
     return any(os.path.getmtime(s) > lib_time for s in _sources())
 
 
+def build_call(force: bool = False) -> str:
+    """Compile the extension module that reads torch tensors for mul and mul_fused (no CUDA code); returns its path.
+    torch is looked up, not imported."""
+    src = os.path.join(CSRC, CALL_SOURCE)
+    if not force and os.path.isfile(CALL_PATH) and os.path.getmtime(CALL_PATH) >= os.path.getmtime(src):
+        return CALL_PATH
+    torch_dir = importlib.util.find_spec("torch").submodule_search_locations[0]
+    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *[f"-isystem{i}" for i in includes], src,
+           "-o", CALL_PATH, "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    subprocess.run(cmd, check=True)
+    return CALL_PATH
+
+
 def build(force: bool = False, verbose: bool = False, trace: bool = False) -> str:
     """Compile every source to an object and link the shared library; returns its path.
     ``trace=True`` builds libfp6m_trace.so instead: the same library with the in-kernel timeline of
     csrc/trace.cuh compiled in (read by ``python -m fp6_marlin_b200.timeline``)."""
+    if not trace:
+        build_call(force)
     lib_path = os.path.join(PKG_DIR, "libfp6m_trace.so") if trace else LIB_PATH
     obj_dir = OBJ_DIR + ("_trace" if trace else "")
     if not force and not trace and not needs_build():

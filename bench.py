@@ -800,7 +800,7 @@ def multi_gpu_extras(env, lb, args, peaks):
 
 def read_traffic_from_profile():
     """DRAM bytes per launch of the GEMM kernel from the committed ncu summary, if one exists."""
-    path = os.path.join(ROOT, "profiles", "w46_gemm_tc5_traffic.json")
+    path = os.path.join(ROOT, "profiles", "w46_gemm_traffic.json")
     if os.path.isfile(path):
         with open(path) as f:
             return json.load(f).get("dram_bytes_per_launch_full_size")

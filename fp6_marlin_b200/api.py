@@ -284,7 +284,7 @@ def launch_plan(m: int, n: int, k: int, quant_cols: int = -1, sms: int = 148):
 # mul
 # ----------------------------------------------------------------------------------------------
 
-_scratch: dict[tuple[int, int], torch.Tensor] = {}
+_scratch: dict[tuple[int, int], list[torch.Tensor]] = {}        # the buffer in use is the last
 _status: dict[int, torch.Tensor] = {}
 _sm_count: dict[int, int] = {}
 _prepared: dict[int, tuple] = {}
@@ -307,7 +307,10 @@ def _device_buffers(device: torch.device, shape=None, stream=None):
 
     The scratch holds the launch epoch and the tagged split-K slots of the kernels, so two GEMMs that
     can overlap on the GPU must not share one: there is one buffer per (device, stream), created (and
-    zeroed, in stream order) the first time a stream is used and grown when a shape needs more.
+    zeroed, in stream order) the first time a stream is used and grown when a shape needs more.  A buffer that
+    a larger one replaces is kept: a call that another thread makes on the stream may have its address and not
+    have launched yet (the native call path runs without the interpreter lock), and a captured graph holds the
+    address for good.  Each is at least twice its predecessor, so all of them are less than twice the last.
     `shape` = (M, N, K, quant_cols) sizes it for that GEMM; None sizes it for any GEMM of up to 16 rows.
     The reference is re-entrant per stream in the same way: each concurrent call brings its own
     workspace (fp6_marlin_cuda_kernel.cu:90-93)."""
@@ -327,14 +330,16 @@ def _device_buffers(device: torch.device, shape=None, stream=None):
             _scratch_need.clear()
         _scratch_need[need_key] = nbytes
     key = (idx, _stream_handle(idx, device) if stream is None else stream)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < nbytes:
+    buffers = _scratch.setdefault(key, [])
+    if not buffers or buffers[-1].numel() < nbytes:
+        if buffers:
+            nbytes = max(nbytes, 2 * buffers[-1].numel())
         # zero once: the kernels keep the epoch and the tagged slots in it between calls
         with torch.cuda.device(device):
             buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        _scratch[key] = buf
+        buffers.append(buf)
         _call.set_scratch(idx, key[1], _ptr(buf), nbytes)
-    return idx, buf, _status[idx]
+    return idx, buffers[-1], _status[idx]
 
 
 def set_launch_overlap(enable: bool) -> bool:

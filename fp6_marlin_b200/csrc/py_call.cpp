@@ -4,7 +4,9 @@
 // attributes and ctypes a call took 11 us, of which the launch itself is about two.  This module handles the calls whose
 // arguments are plain CUDA tensors that pass every check; for anything else - subclasses, wrappers of function
 // transforms, wrong sizes or types - it answers "not handled" and the caller takes its general path, which raises or
-// computes as before.  It holds no state but the scratch buffers registered by the caller (one per device and stream).
+// computes as before.  It holds no state but the addresses of the scratch buffers registered by the caller (one per device and
+// stream); the caller never frees a registered buffer, also not one that a larger one replaces: a call may have read its
+// address here and not have launched yet.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
@@ -158,7 +160,7 @@ PyObject* py_set_device(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
-// set_scratch(dev, stream, address, bytes); the caller keeps the memory alive
+// set_scratch(dev, stream, address, bytes); the caller keeps the memory for the life of the process
 PyObject* py_set_scratch(PyObject*, PyObject* args) {
   int dev;
   unsigned long long stream, ptr, bytes;

@@ -13,6 +13,7 @@ PyTorch is used for memory, streams and device management only.
 from __future__ import annotations
 
 import ctypes
+import threading
 import weakref
 
 import torch
@@ -287,6 +288,7 @@ def launch_plan(m: int, n: int, k: int, quant_cols: int = -1, sms: int = 148):
 _scratch: dict[tuple[int, int], list[torch.Tensor]] = {}        # the buffer in use is the last
 _status: dict[int, torch.Tensor] = {}
 _sm_count: dict[int, int] = {}
+_buffers_lock = threading.RLock()          # (reentrant: an allocation may run a finalizer)
 _prepared: dict[int, tuple] = {}
 
 
@@ -315,31 +317,34 @@ def _device_buffers(device: torch.device, shape=None, stream=None):
     The reference is re-entrant per stream in the same way: each concurrent call brings its own
     workspace (fp6_marlin_cuda_kernel.cu:90-93)."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    if idx not in _status:
-        _status[idx] = torch.zeros(1, dtype=torch.int32, device=device)
-        _sm_count[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-        _call.set_device(idx, _ptr(_status[idx]), _sm_count[idx])
-    need_key = (idx, shape)
-    nbytes = _scratch_need.get(need_key)
-    if nbytes is None:
-        if shape is None:
-            nbytes = lib.fp6m_mul_scratch_bytes(16, 1 << 20, 1 << 14, 0, _sm_count[idx])
-        else:
-            nbytes = lib.fp6m_mul_scratch_bytes(shape[0], shape[1], shape[2], shape[3], _sm_count[idx])
-        if len(_scratch_need) > 4096:
-            _scratch_need.clear()
-        _scratch_need[need_key] = nbytes
-    key = (idx, _stream_handle(idx, device) if stream is None else stream)
-    buffers = _scratch.setdefault(key, [])
-    if not buffers or buffers[-1].numel() < nbytes:
-        if buffers:
-            nbytes = max(nbytes, 2 * buffers[-1].numel())
-        # zero once: the kernels keep the epoch and the tagged slots in it between calls
-        with torch.cuda.device(device):
-            buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        buffers.append(buf)
-        _call.set_scratch(idx, key[1], _ptr(buf), nbytes)
-    return idx, buffers[-1], _status[idx]
+    # One thread at a time: an allocation lets others run, and two that both made the buffer of a stream, or the status word of a
+    # device, would register them in an order of their own and drop one that the native call path goes on using.
+    with _buffers_lock:
+        if idx not in _status:
+            _status[idx] = torch.zeros(1, dtype=torch.int32, device=device)
+            _sm_count[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
+            _call.set_device(idx, _ptr(_status[idx]), _sm_count[idx])
+        need_key = (idx, shape)
+        nbytes = _scratch_need.get(need_key)
+        if nbytes is None:
+            if shape is None:
+                nbytes = lib.fp6m_mul_scratch_bytes(16, 1 << 20, 1 << 14, 0, _sm_count[idx])
+            else:
+                nbytes = lib.fp6m_mul_scratch_bytes(shape[0], shape[1], shape[2], shape[3], _sm_count[idx])
+            if len(_scratch_need) > 4096:
+                _scratch_need.clear()
+            _scratch_need[need_key] = nbytes
+        key = (idx, _stream_handle(idx, device) if stream is None else stream)
+        buffers = _scratch.setdefault(key, [])
+        if not buffers or buffers[-1].numel() < nbytes:
+            if buffers:
+                nbytes = max(nbytes, 2 * buffers[-1].numel())
+            # zero once: the kernels keep the epoch and the tagged slots in it between calls
+            with torch.cuda.device(device):
+                buf = torch.zeros(nbytes, dtype=torch.uint8, device=device)
+            buffers.append(buf)
+            _call.set_scratch(idx, key[1], _ptr(buf), nbytes)
+        return idx, buffers[-1], _status[idx]
 
 
 def set_launch_overlap(enable: bool) -> bool:

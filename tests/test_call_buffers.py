@@ -1,6 +1,7 @@
 """The buffers that calls of `mul` share - a split-K scratch per (device, stream), a status word per device - as the host keeps
 them, with tensors in host memory and a recorder in the place of the native call path (nothing here reaches a GPU)."""
 import contextlib
+import threading
 import types
 import weakref
 
@@ -46,3 +47,27 @@ def test_replaced_scratches_are_bounded(registered):
             _, last, _ = api._device_buffers(DEV, (m, n, 4096, 0), STREAM)
     buffers = api._scratch[63, STREAM]
     assert buffers[-1] is last and sum(b.numel() for b in buffers) < 2 * last.numel()
+
+
+def test_first_calls_of_two_threads_share_their_buffers(registered, monkeypatch):
+    """Both threads reach the allocations of a stream's first call together (as far as they are let): one scratch and one status
+    word are made, and what is registered is what both use."""
+    together, zeros = threading.Barrier(2), torch.zeros
+    made, got = [], []
+
+    def slow_zeros(*args, **kw):
+        with contextlib.suppress(threading.BrokenBarrierError):
+            together.wait(0.3)
+        made.append(zeros(*args, **kw))
+        return made[-1]
+
+    monkeypatch.setattr(torch, "zeros", slow_zeros)
+    threads = [threading.Thread(target=lambda: got.append(api._device_buffers(DEV, SMALL, STREAM))) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(made) == 2 and len(registered) == 2
+    (_, scratch, status), (_, other_scratch, other_status) = got
+    assert scratch is other_scratch and status is other_status
+    assert dict(registered) == {"device": (63, status.data_ptr(), 148), "scratch": (63, STREAM, scratch.data_ptr(), scratch.numel())}

@@ -119,3 +119,35 @@ def test_captured_graph_keeps_its_scratch(layer):
     torch.cuda.synchronize()
     assert all(bool((o == 0x5A).all()) for o in others)
     assert fm.device_status(dev) == 0
+
+
+@pytest.mark.parametrize("attempt", range(3))
+def test_first_calls_of_threads_on_one_stream(layer, attempt):
+    """Nobody has made the stream's scratch when eight threads call at once, with rows that need scratches of four sizes."""
+    dev = layer.B.device
+    rows = [1, 8, 16, 20, 33, 64, 100, 300]
+    inputs = [synth.make_activations(m, K, m).to(dev) for m in rows]
+    ordered = fm.set_ordered_sums(True)
+    want = [_mul(layer, a) for a in inputs]
+    stream, go = torch.cuda.Stream(dev), threading.Barrier(len(rows))
+    torch.cuda.synchronize()
+    results, failures = {}, []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(stream):
+                go.wait()
+                results[i] = [_mul(layer, inputs[i]) for _ in range(5)]
+        except Exception as e:
+            failures.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(rows))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    fm.set_ordered_sums(ordered)
+    assert not failures, failures
+    assert all(torch.equal(c, want[i]) for i in results for c in results[i])
+    assert fm.device_status(dev) == 0

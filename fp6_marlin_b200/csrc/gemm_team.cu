@@ -56,7 +56,28 @@ struct TeamCfg {
   static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   static constexpr int kOutTeams = T < 4 ? 2 : 4;      // teams that write finished rows
   static constexpr int kOutRows = NT / kOutTeams;
+  // Up to 32 rows a strip that goes on in other CTAs is summed by all teams and the four warps before them (issuers that are done),
+  // eight rows a thread, so that add_partials has two contributors in flight per round trip to L2.  Measured against the two output
+  // teams alone (sixteen rows a thread, one contributor per round trip), us at 32 rows: 16384 x 1024 18.2 -> 14.2,
+  // 8192 x 2048 12.7 -> 10.8, 4096 x 1024 9.6 -> 9.0, 4096 x 4096 9.9 -> 9.5, 8192 x 57344 and 8192 x 28672 equal.  (Two contributors with
+  // sixteen rows a thread spill: 8192 x 2048 13.7, K = N = 8192 17.3 instead of 15.2.)  With sixteen rows the output teams have
+  // eight a thread anyway.
+  static constexpr int kSumGroups = NT > 16 ? 4 : kOutTeams;
+  static constexpr int kSumRows = NT / kSumGroups;
+  static constexpr bool kSumHelpers = kSumGroups > T;
+  static_assert(kSumGroups <= T + 1 && kTeamBase - 4 >= kIssueBase, "one group of helpers, and none of them a producer");
 };
+
+// the sums of the teams for the rows row0 ... of column c
+template <class C, int RR>
+__device__ __forceinline__ void pooled_sums(uint32_t pool, int row0, int c, float (&out)[RR]) {
+#pragma unroll
+  for (int m = 0; m < RR; ++m) {
+    out[m] = 0.f;
+#pragma unroll
+    for (int e = 0; e < C::T; ++e) out[m] += lds_f32(pool + ((e * C::NT + row0 + m) * kStripCols + c) * 4);
+  }
+}
 
 template <class C>
 __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __grid_constant__ MulParams p, const __grid_constant__ CUtensorMap amap) {
@@ -256,16 +277,12 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
       named_bar_sync(1, C::kTeamThreads);        // the sums of the slice before have been read
 #pragma unroll
       for (int m = 0; m < NT; ++m) sts_f32(pool + ((team * NT + m) * kStripCols + c) * 4, acc[m]);
+      if (C::kSumHelpers && b0 == 0 && b1 < kb) return;      // at the kernel's end, with the helpers
       named_bar_sync(1, C::kTeamThreads);
       if (team >= C::kOutTeams) return;
       constexpr int RR = C::kOutRows;
       float out[RR];
-#pragma unroll
-      for (int m = 0; m < RR; ++m) {
-        out[m] = 0.f;
-#pragma unroll
-        for (int e = 0; e < T; ++e) out[m] += lds_f32(pool + ((e * NT + row0 + m) * kStripCols + c) * 4);
-      }
+      pooled_sums<C>(pool, row0, c, out);
       uint32_t tag = 0;
       if (b0 > 0 || b1 < kb) {
         mbar_wait(epoch_bar, 0, ws);
@@ -276,11 +293,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
         return;
       }
       if (b1 < kb) add_partials<RR>(p, cta, (s + 1) * kb, NT, row0, c, tag, out, ws);
-      const bool writes = c < strip_cols(is6 ? geo.n6 : geo.n4, strip);
-      const float col_scale = strip_column_scale(p, is6, strip, c, writes);
-#pragma unroll
-      for (int m = 0; m < RR; ++m) out[m] *= col_scale;
-      store_column_rows<RR>(p, row0, is6, strip * kStripCols + c, out, writes);
+      finish_column_rows<RR>(p, row0, is6, strip, c, out);
     };
     auto add_sums = [&](uint32_t d, uint32_t scale_raw) {
       const float scale = __half2float(__ushort_as_half((unsigned short)scale_raw));
@@ -361,6 +374,23 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
 #pragma unroll
       for (int m = 0; m < NT; ++m) acc[m] = 0.f;
       ++cur;
+    }
+  }
+  if constexpr (C::kSumHelpers) {
+    const int s = (B1 - 1) / kb;
+    if (warp >= C::kTeamBase - 4 && (s > s_first || blk_first == 0) && B1 < (s + 1) * kb) {
+      // the CTA's last strip starts here and goes on in the next CTA; the teams have left their sums of it in the pool
+      named_bar_sync(2, C::kTeamThreads + 128);
+      const int group = warp >= C::kTeamBase ? (warp - C::kTeamBase) >> 2 : T;
+      constexpr int RR = C::kSumRows;
+      const int row0 = group * RR, c = (warp & 3) * 32 + lane;
+      const bool is6 = s >= geo.strips4;
+      const int strip = is6 ? s - geo.strips4 : s;
+      float out[RR];
+      pooled_sums<C>(pool, row0, c, out);
+      mbar_wait(epoch_bar, 0, ws);
+      add_partials<RR>(p, cta, (s + 1) * kb, NT, row0, c, misc[1] + 1, out, ws);
+      finish_column_rows<RR>(p, row0, is6, strip, c, out);
     }
   }
   report_waits(ws, p.status);

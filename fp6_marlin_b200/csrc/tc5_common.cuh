@@ -413,5 +413,14 @@ __device__ __forceinline__ float strip_column_scale(const Params& p, bool is6, i
   const half* sp = p.S + (is6 ? fp6_scale_offset(p.geo, strip) : int4_scale_offset(p.geo, strip, 0));
   return __half2float(__ldg(sp + c)) * (is6 ? 4096.f : 1.f);
 }
+// finished sums of column c of a strip, rows row0 ...: column scale, one rounding, store
+template <int RR, class Params>
+__device__ __forceinline__ void finish_column_rows(const Params& p, int row0, bool is6, int strip, int c, float (&out)[RR]) {
+  const bool writes = c < strip_cols(is6 ? p.geo.n6 : p.geo.n4, strip);
+  const float col_scale = strip_column_scale(p, is6, strip, c, writes);
+#pragma unroll
+  for (int m = 0; m < RR; ++m) out[m] *= col_scale;
+  store_column_rows<RR>(p, row0, is6, strip * kStripCols + c, out, writes);
+}
 
 }  // namespace fp6m

@@ -5,6 +5,7 @@ work before the package itself can be imported)
 """
 from __future__ import annotations
 
+import hashlib
 import importlib.util
 import os
 import shutil
@@ -16,7 +17,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libfp6m.so")
 CALL_PATH = os.path.join(PKG_DIR, "_call.so")          # extension module: the Python call path of mul and mul_fused
-CALL_SOURCE = "py_call.cpp"
+CALL_SOURCES = [os.path.join(CSRC, "py_call.cpp"), os.path.join(os.path.dirname(PKG_DIR), "include", "fp6m.h")]
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 
 CUDA_SOURCES = ["c_api.cu", "gemm_few.cu", "gemm_team.cu", "gemm_tc5.cu", "gemm_wide.cu", "dump_operands.cu", "prep_gpu.cu", "gather_columns.cu", "peer.cu"]
@@ -47,19 +48,41 @@ def needs_build() -> bool:
     return any(os.path.getmtime(s) > lib_time for s in _sources())
 
 
-def build_call(force: bool = False) -> str:
-    """Compile the extension module that reads torch tensors for mul and mul_fused (no CUDA code); returns its path.
-    torch is looked up, not imported."""
-    src = os.path.join(CSRC, CALL_SOURCE)
-    if not force and os.path.isfile(CALL_PATH) and os.path.getmtime(CALL_PATH) >= os.path.getmtime(src):
-        return CALL_PATH
-    torch_dir = importlib.util.find_spec("torch").submodule_search_locations[0]
+def _torch_dir() -> str:
+    """Where torch is installed (looked up, not imported)."""
+    return importlib.util.find_spec("torch").submodule_search_locations[0]
+
+
+def _call_command() -> list[str]:
+    torch_dir = _torch_dir()
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
                 os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *[f"-isystem{i}" for i in includes], src,
-           "-o", CALL_PATH, "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
-    subprocess.run(cmd, check=True)
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *[f"-isystem{i}" for i in includes],
+            CALL_SOURCES[0], "-o", CALL_PATH, "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+
+
+def _call_stamp() -> str:
+    """What the extension module depends on: its sources (the C ABI's declarations among them), the command, this Python, and torch,
+    whose accessors it has inlined and whose fields it reads at their offsets."""
+    digest = hashlib.sha256("\0".join([sys.version, *_call_command()]).encode())
+    for path in [*CALL_SOURCES, os.path.join(_torch_dir(), "version.py")]:
+        with open(path, "rb") as f:
+            digest.update(f.read())
+    return digest.hexdigest()
+
+
+def build_call(force: bool = False) -> str:
+    """Compile the extension module that reads torch tensors for mul and mul_fused (no CUDA code); returns its path."""
+    stamp_path, stamp = os.path.join(OBJ_DIR, "_call.stamp"), _call_stamp()
+    if not force and os.path.isfile(CALL_PATH) and os.path.isfile(stamp_path):
+        with open(stamp_path) as f:
+            if f.read() == stamp:
+                return CALL_PATH
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    subprocess.run(_call_command(), check=True)
+    with open(stamp_path, "w") as f:
+        f.write(stamp)
     return CALL_PATH
 
 

@@ -16,21 +16,19 @@
 #include <cstdint>
 #include <unordered_map>
 
+#include "../../include/fp6m.h"
+
 namespace {
 
-typedef int (*MulFn)(const void* A, const void* B, void* C, const void* s, int M, int N, int K, void* workspace, size_t workspace_bytes,
-                     void* scratch, size_t scratch_bytes, int dev, void* stream, int thread_k, int thread_n, int sms, int max_par,
-                     int quant_cols, int group_size, int layout, int* status_dev);
-typedef int (*MulFusedFn)(const void* A, const void* B, void* C, const void* s, int M, int N, int K, void* workspace, size_t workspace_bytes,
-                          void* scratch, size_t scratch_bytes, int dev, void* stream, int thread_k, int thread_n, int sms, int max_par,
-                          int quant_cols, int group_size, int layout, int* status_dev, int epilogue, const void* residual);
-typedef size_t (*ScratchFn)(int M, int N, int K, int quant_cols, int sms);
+// (the types of the C ABI's own declarations: the addresses come as numbers, see bind)
+using MulFn = decltype(&fp6m_mul);
+using MulFusedFn = decltype(&fp6m_mul_fused);
+using ScratchFn = decltype(&fp6m_mul_scratch_bytes);
 
 MulFn g_mul = nullptr;
 MulFusedFn g_mul_fused = nullptr;
 ScratchFn g_scratch_bytes = nullptr;
 
-constexpr int kLayoutB200 = 1, kEpilogueSiluMul = 1, kEpilogueResidual = 2;
 constexpr long kNotHandled = -1;
 
 // What the caller registered (all access under the interpreter lock).
@@ -92,12 +90,12 @@ PyObject* mul_impl(PyObject* const* args) {
       !as_int(args[8], &sms) || !as_int(args[9], &max_par) || !as_int(args[10], &group_size) || !as_int(args[11], &epilogue))
     return PyLong_FromLong(kNotHandled);
   if (A->dim() != 2 || C->dim() != 2) return PyLong_FromLong(kNotHandled);
-  const int64_t M = A->size(0), K = A->size(1), N = C->size(1) * (epilogue == kEpilogueSiluMul ? 2 : 1);
+  const int64_t M = A->size(0), K = A->size(1), N = C->size(1) * (epilogue == FP6M_EPILOGUE_SILU_MUL ? 2 : 1);
   if (M <= 0 || K <= 0 || N <= 0 || M > INT32_MAX || K > INT32_MAX || N > INT32_MAX || C->size(0) != M || max_par < 1) return PyLong_FromLong(kNotHandled);
   if (ws->numel() < N / 128 * max_par) return PyLong_FromLong(kNotHandled);
   if (A->scalar_type() != at::kHalf || C->scalar_type() != at::kHalf || s->scalar_type() != at::kHalf) return PyLong_FromLong(kNotHandled);
   const void* residual = nullptr;
-  if (epilogue == kEpilogueResidual) {
+  if (epilogue == FP6M_EPILOGUE_RESIDUAL) {
     const at::Tensor* r = plain_cuda(args[12]);
     if (!r || r->scalar_type() != at::kHalf || r->dim() != 2 || r->size(0) != M || r->size(1) != N) return PyLong_FromLong(kNotHandled);
     residual = r->data_ptr();
@@ -117,10 +115,10 @@ PyObject* mul_impl(PyObject* const* args) {
   Py_BEGIN_ALLOW_THREADS        // a launch waits while the GPU's queue is full
   if (epilogue)
     rc = g_mul_fused(a, w, c, sc, (int)M, (int)N, (int)K, wsp, ws_bytes, scratch.ptr, scratch.bytes, dev, stream, thread_k, thread_n, sms, max_par,
-                     quant_cols, group_size, kLayoutB200, status, epilogue, residual);
+                     quant_cols, group_size, FP6M_LAYOUT_B200, status, epilogue, residual);
   else
     rc = g_mul(a, w, c, sc, (int)M, (int)N, (int)K, wsp, ws_bytes, scratch.ptr, scratch.bytes, dev, stream, thread_k, thread_n, sms, max_par,
-               quant_cols, group_size, kLayoutB200, status);
+               quant_cols, group_size, FP6M_LAYOUT_B200, status);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
 }

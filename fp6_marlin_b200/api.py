@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
+import warnings
 import weakref
 
 import torch
@@ -22,11 +23,40 @@ from torch.autograd import forward_ad
 from . import _lib
 from ._lib import lib
 
-try:
-    from . import _call
-except ImportError as e:
-    raise ImportError(f"fp6_marlin_b200/_call.so is missing or does not load ({e}): build it with `python fp6_marlin_b200/build.py`") from e
 
+class _GeneralPathOnly:
+    """In the place of the extension module ``_call`` where that is missing or does not fit this torch: ``mul`` and ``mul_fused`` take
+    their general path, which does the same at about 5 us more of host time per call; nothing else needs the module."""
+
+    def __init__(self, reason):
+        self.reason = reason
+
+    def bind(self, *addresses):
+        pass
+
+    def set_scratch(self, *buffer):
+        pass
+
+    def set_device(self, *device):            # once per device, by its first GEMM
+        warnings.warn(f"fp6_marlin_b200: calls take the slower general path, because {self.reason}; build with "
+                      "`python fp6_marlin_b200/build.py`", RuntimeWarning, stacklevel=4)
+
+    def mul(self, *args):
+        return -1                             # not handled
+
+
+def _native_call_path():
+    try:
+        from . import _call
+    except ImportError as e:
+        return _GeneralPathOnly(f"fp6_marlin_b200/_call.so is missing or does not load ({e})")
+    built_for = getattr(_call, "torch_version", None)
+    if built_for != str(torch.__version__):           # it reads tensors at the offsets of the headers it was compiled with
+        return _GeneralPathOnly(f"fp6_marlin_b200/_call.so was built for torch {built_for}, this is {torch.__version__}")
+    return _call
+
+
+_call = _native_call_path()
 _call.bind(*(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in ("fp6m_mul", "fp6m_mul_fused", "fp6m_mul_scratch_bytes")))
 
 

@@ -8,6 +8,7 @@ from __future__ import annotations
 import hashlib
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -58,7 +59,9 @@ def _call_command() -> list[str]:
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
                 os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
-    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *[f"-isystem{i}" for i in includes],
+    with open(os.path.join(torch_dir, "version.py")) as f:
+        version = re.search(r"^__version__ = '([^']+)'", f.read(), re.M).group(1)
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f'-DFP6M_TORCH_VERSION="{version}"', *[f"-isystem{i}" for i in includes],
             CALL_SOURCES[0], "-o", CALL_PATH, "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
 
 

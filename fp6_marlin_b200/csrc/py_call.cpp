@@ -181,4 +181,9 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_call", "host call path of mul an
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__call(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__call(void) {
+  PyObject* module = PyModule_Create(&kModule);
+  // the importer compares it with the torch it has: torch's accessors are inlined here
+  if (module && PyModule_AddStringConstant(module, "torch_version", FP6M_TORCH_VERSION) != 0) Py_CLEAR(module);
+  return module;
+}

@@ -185,7 +185,7 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
   // a caller's fixed scratch (fp6m_mul_static_scratch) may hold the partials of the fewest tiles only
   if (scratch_bytes < scratch_bytes_of(lp)) lp = plan_launches(M, p.geo, sms, -1, true);
   const bool wide = lp.wide;
-  const int tile = lp.tile, rows = lp.rows, ctas = lp.ctas;
+  const int rows = lp.rows, ctas = lp.ctas;
   if (scratch_bytes < scratch_bytes_of(lp)) return FP6M_ERR_SCRATCH;
   p.B = static_cast<const uint8_t*>(B);
   p.S = static_cast<const half*>(s);

@@ -38,6 +38,11 @@ struct TeamCfg {
   static constexpr int T = TEAMS_;
   static constexpr int kStages = STAGES_;
   static_assert(kStages % T == 0, "a stage always belongs to the same team");
+  // The two weights producers take every second segment, so with an odd number of stages a stage changes producer on each use, and
+  // a producer waits for every second phase of w_empty only.  Its parity wait for segment n - S must not pass on the phase before,
+  // so segment n - 2 S must have been read by then.  It has: this producer has waited for segment n - 2 T - S, which the same
+  // team reads, in order, and which is not before n - 2 S.
+  static_assert(2 * T <= kStages, "a weights producer's waits bound the phase of a stage");
   static_assert(kStages <= 32, "the first round of weight copies is issued by one lane per stage");
   static constexpr int kIssueBase = 3;                 // warps 0, 1: weights; 2: activations, TMEM, epoch; then one MMA issuer per team
   static constexpr int kTeamBase = (kIssueBase + T + 3) & ~3;
@@ -194,7 +199,9 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
     }
   } else if (warp == 2) {
     // ================================================================== activations producer; launch epoch
-    const bool act3d = (p.K & 63) == 0;        // the host encoded the three-dimensional map
+    // The host encoded the three-dimensional map.  (It does for every K that mul_impl lets through, multiples of 64; without the
+    // other branch the 16-row instance measures slower: 8192 x 28672 at 9 rows 33.7 -> 34.2 us, 16384 x 1024 12.3 -> 12.45.)
+    const bool act3d = (p.K & 63) == 0;
     int blk = blk_first, r = 0;
     uint32_t phase = 1;                        // a fresh barrier passes parity 1
     for (int n = 0; n < nseg; ++n) {

@@ -204,10 +204,8 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     for (int q = 0; q < out.n_out; ++q) ok = ok && aligned16(out.peer[q]);
     p.vec_rows = ok ? 1 : 0;
   }
-  // The kernel for 33 to 128 rows may also expand its first segments before the grid dependency resolves (measured -2 to -3 %
-  // on a chain of launches).
   p.weights_early = tc5_get_overlap() ? 1 : 0;
-  p.expand_early = (p.weights_early && !wide) ? 1 : 0;
+  const long long blocks = (long long)(p.geo.strips4 + p.geo.strips6) * p.geo.k128;
 
   for (int m0 = 0; m0 < M; m0 += rows) {
     p.A = static_cast<const half*>(A) + (size_t)m0 * K;
@@ -224,6 +222,11 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     p.tile_rows = launch_wide ? wide_tile_rows(p.M, p.row_tiles) : 0;
     make_schedule(p.geo, launch_ctas, &p.sched, p.row_tiles, !launch_wide && p.M <= kTeamMaxRows ? 0 : kReducerPenalty);
     align_schedule_to_blocks(&p.sched);
+    // The kernels for 9 to 128 rows may also expand their first segments before the grid dependency resolves: above 32 rows always
+    // (measured -2 to -3 % on a chain of launches), up to 32 rows with at most 20 blocks per CTA: us at 16 / 32 rows 4096 x 4096 (8 blocks) 7.73 /
+    // 9.38 -> 6.97 / 8.57, 4096 x 1024 7.33 / 8.74 -> 6.88 / 8.14, 11008 x 4096 (19) 11.2 / 12.8 -> 11.1 / 12.6, but K = N = 8192 (28) 12.77 / 14.4
+    // -> 12.70 / 14.3 and 8192 x 28672 (97) 32.5 / 35.3 -> 32.2 / 35.6: there the next launch's CTAs get their SMs too late for it.
+    p.expand_early = (p.weights_early && !wide && (p.M > kTeamMaxRows || blocks <= 20ll * launch_ctas)) ? 1 : 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // the lines between the kernels: measured at 5, 8, 16 and 32 rows, see the heads of gemm_few.cu and gemm_team.cu
     cudaError_t e = launch_wide ? launch_gemm_wide(p, st)

@@ -48,7 +48,7 @@ struct MulParams {
   int* status;          // optional device status word
   OutputMap out;
   int weights_early;    // the kernel before this one in the stream does not write B or S: read them before it has finished
-  int expand_early;     // (only with weights_early) kernel for 33 to 128 rows: the teams expand their first segments before the grid dependency
+  int expand_early;     // (only with weights_early) kernels for 9 to 128 rows: the teams expand their first segments before the grid dependency
   int vec_rows;         // kernel for more than 128 rows: finished rows leave as 16-byte stores (every row start and both
                         // column bases are multiples of 8 halves, no fused epilogue)
   int tile_rows;        // kernel for more than 128 rows: rows of a tile

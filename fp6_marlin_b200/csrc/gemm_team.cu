@@ -84,7 +84,7 @@ __device__ __forceinline__ void pooled_sums(uint32_t pool, int row0, int c, floa
   }
 }
 
-template <class C>
+template <class C, bool EARLY>
 __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __grid_constant__ MulParams p, const __grid_constant__ CUtensorMap amap) {
   constexpr int NT = C::NT, S = C::kStages, T = C::T;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -160,7 +160,9 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, misc[0], 0);      // uniform to the compiler
-  grid_dependency_wait();
+  // With EARLY (p.expand_early) the teams go on: their first segments need the weights only.  An instance of its own, because as a
+  // condition it costs the calls without it 0.03 us.
+  if (!EARLY || warp < C::kTeamBase) grid_dependency_wait();
 
   if (warp < 2) {
     // ================================================================== weights producers: every other segment each
@@ -359,6 +361,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(rd + 8);
+      if constexpr (EARLY) grid_dependency_wait();       // before the first wait for an MMA, and before anything is written
       if (i > 0) add_sums(d0 + ((i - 1) & 1) * NT, scale_prev);
       while (cur < s) {
         finish();
@@ -370,6 +373,7 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
       stage += T;
       if (stage >= S) { stage -= S; wphase ^= 1; }
     }
+    if constexpr (EARLY) grid_dependency_wait();         // (a team without segments)
     if (i > 0) {
       mbar_wait(fr + 8, (i - 1) & 1, ws);
       tc_fence_after();
@@ -412,13 +416,13 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
 using Team16 = TeamCfg<16, 12, 3>;
 using Team32 = TeamCfg<32, 9, 3>;
 
-template <class C>
+template <class C, bool EARLY>
 cudaError_t launch_team(const MulParams& p, cudaStream_t stream) {
   static std::atomic<bool> configured[64] = {};       // threads that find it false set the same attribute
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(w46_gemm_team_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(w46_gemm_team_kernel<C, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
@@ -436,13 +440,14 @@ cudaError_t launch_team(const MulParams& p, cudaStream_t stream) {
   cudaError_t me = (p.K & 63) == 0 ? encode_activation_segment_map(p.A, p.M, p.K, C::NT, &amap)
                                    : encode_activation_map(p.A, p.M, p.K, C::NT, &amap);
   if (me != cudaSuccess) return me;
-  return cudaLaunchKernelEx(&cfg, w46_gemm_team_kernel<C>, p, amap);
+  return cudaLaunchKernelEx(&cfg, w46_gemm_team_kernel<C, EARLY>, p, amap);
 }
 
 }  // namespace
 
 cudaError_t launch_gemm_team(const MulParams& p, cudaStream_t stream) {
-  return p.M <= 16 ? launch_team<Team16>(p, stream) : launch_team<Team32>(p, stream);
+  if (p.M <= 16) return p.expand_early ? launch_team<Team16, true>(p, stream) : launch_team<Team16, false>(p, stream);
+  return p.expand_early ? launch_team<Team32, true>(p, stream) : launch_team<Team32, false>(p, stream);
 }
 
 }  // namespace fp6m

@@ -32,7 +32,7 @@ namespace fp6m {
 
 namespace {
 
-template <int NT_, int STAGES_, int TEAMS_>
+template <int NT_, int STAGES_, int TEAMS_, int SUM_GROUPS_>
 struct TeamCfg {
   static constexpr int NT = NT_;                       // rows of A = N of the MMA
   static constexpr int T = TEAMS_;
@@ -61,13 +61,11 @@ struct TeamCfg {
   static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   static constexpr int kOutTeams = T < 4 ? 2 : 4;      // teams that write finished rows
   static constexpr int kOutRows = NT / kOutTeams;
-  // Up to 32 rows a strip that goes on in other CTAs is summed by all teams and the four warps before them (issuers that are done),
-  // eight rows a thread, so that add_partials has two contributors in flight per round trip to L2.  Measured against the two output
-  // teams alone (sixteen rows a thread, one contributor per round trip), us at 32 rows: 16384 x 1024 18.2 -> 14.2,
-  // 8192 x 2048 12.7 -> 10.8, 4096 x 1024 9.6 -> 9.0, 4096 x 4096 9.9 -> 9.5, 8192 x 57344 and 8192 x 28672 equal.  (Two contributors with
-  // sixteen rows a thread spill: 8192 x 2048 13.7, K = N = 8192 17.3 instead of 15.2.)  With sixteen rows the output teams have
-  // eight a thread anyway.
-  static constexpr int kSumGroups = NT > 16 ? 4 : kOutTeams;
+  // Groups of four warps that sum a strip which goes on in other CTAs, with their shares of the rows: 2 = the output teams, 4 = all teams
+  // and the four warps before them (issuers that are done).  More groups mean fewer rows a thread and so more contributors in flight
+  // per round trip to L2 (add_partials): with 16 rows four instead of two, with 32 rows two instead of one.  (Two with the sixteen rows a
+  // thread of two groups spill: 8192 x 2048 at 32 rows 13.7 us, K = N = 8192 17.3 instead of 15.2.)  launch_gemm_team says which is when faster.
+  static constexpr int kSumGroups = SUM_GROUPS_;
   static constexpr int kSumRows = NT / kSumGroups;
   static constexpr bool kSumHelpers = kSumGroups > T;
   static_assert(kSumGroups <= T + 1 && kTeamBase - 4 >= kIssueBase, "one group of helpers, and none of them a producer");
@@ -413,11 +411,13 @@ __global__ void __launch_bounds__(C::kThreads, 1) w46_gemm_team_kernel(const __g
   }
 }
 
-using Team16 = TeamCfg<16, 12, 3>;
-using Team32 = TeamCfg<32, 9, 3>;
+using Team16 = TeamCfg<16, 12, 3, 2>;
+using Team16Cut = TeamCfg<16, 12, 3, 4>;
+using Team32 = TeamCfg<32, 9, 3, 2>;
+using Team32Cut = TeamCfg<32, 9, 3, 4>;
 
 template <class C, bool EARLY>
-cudaError_t launch_team(const MulParams& p, cudaStream_t stream) {
+cudaError_t launch_instance(const MulParams& p, cudaStream_t stream) {
   static std::atomic<bool> configured[64] = {};       // threads that find it false set the same attribute
   int dev = 0;
   cudaGetDevice(&dev);
@@ -443,11 +443,22 @@ cudaError_t launch_team(const MulParams& p, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, w46_gemm_team_kernel<C, EARLY>, p, amap);
 }
 
+template <class C>
+cudaError_t launch_team(const MulParams& p, cudaStream_t stream) {
+  return p.expand_early ? launch_instance<C, true>(p, stream) : launch_instance<C, false>(p, stream);
+}
+
 }  // namespace
 
 cudaError_t launch_gemm_team(const MulParams& p, cudaStream_t stream) {
-  if (p.M <= 16) return p.expand_early ? launch_team<Team16, true>(p, stream) : launch_team<Team16, false>(p, stream);
-  return p.expand_early ? launch_team<Team32, true>(p, stream) : launch_team<Team32, false>(p, stream);
+  // Four groups pay where strips are cut over many CTAs.  Up to 16 rows that is at least four on average (us at 16 rows, two groups -> four:
+  // sixteen CTAs per strip 16384 x 1024 12.2 -> 10.5, nine 11008 x 2048 10.1 -> 9.5, eight 8192 x 2048 9.2 -> 8.8, four 4096 x 1024 7.70 -> 7.65
+  // and 4096 x 4096 equal, but 2.3 K = N = 8192 13.3 -> 13.6, 1.5 4096 x 12288 11.4 -> 11.9, one 1024 x 1024 6.4 -> 6.7); up to 32 rows more than
+  // one (at 32 rows sixteen 18.3 -> 14.2, eight 12.7 -> 10.8, four 9.6 -> 9.0 and 9.9 -> 9.5, 2.3 15.2 -> 15.1, 1.5 13.0 -> 12.9, but one 7.39 -> 7.44
+  // and 0.7 8192 x 28672 36.3 -> 36.5).
+  const int ctas = p.sched.ctas, strips = p.geo.strips4 + p.geo.strips6;
+  if (p.M > 16) return ctas > strips ? launch_team<Team32Cut>(p, stream) : launch_team<Team32>(p, stream);
+  return ctas >= 4 * strips ? launch_team<Team16Cut>(p, stream) : launch_team<Team16>(p, stream);
 }
 
 }  // namespace fp6m

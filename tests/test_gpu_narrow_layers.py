@@ -1,8 +1,8 @@
-"""17 to 32 rows on layers whose strips are cut over many CTAs: all teams and the warps before them sum a strip (gemm_team.cu).
+"""9 to 32 rows on layers whose strips are cut over many CTAs: all teams and the warps before them sum a strip (gemm_team.cu).
 
-Bound of the values: as in test_gpu_few_rows.py.  Bound of the time: a call of 32 rows reads and sums twice the partials of a call of 16
-and streams the same weights, which are most of it; summing with two teams and one contributor per round trip made it 1.5 times as
-long (18.3 against 12.2 us for 16384 x 1024), with the warps of four groups it is 1.17 times.  1.35 is asserted."""
+Bound of the values: as in test_gpu_few_rows.py.  Bound of the time: against 8 rows, which another kernel serves, a call reads and sums two and four times the partials and streams the
+same weights, which are most of it.  On 16384 x 1024 summing with two teams took 1.36 times the time at 16 rows and 2.0 times at 32
+(9.1, 12.4 and 18.3 us), with four groups of warps 1.17 and 1.56 times; 1.27 and 1.75 are asserted."""
 import pytest
 import torch
 
@@ -22,7 +22,7 @@ def test_sums_of_shared_strips(qc, group, sms):
     w = synth.make_layer(K, N, qc, group, seed=sms, keep_dequantized=False).to(dev)
     w64 = fm.dump_operands(w.B, w.s, K, N, qc, group).double()
     workspace = torch.zeros(N // 128 * 16, dtype=torch.int32, device=dev)
-    for m in (17, 24, 25, 32):
+    for m in (9, 13, 16, 17, 24, 25, 32):
         a = synth.make_activations(m, K, m).to(dev)
         ref = a.double() @ w64
         c = torch.full((m + 1, N), 3.0, dtype=torch.float16, device=dev)
@@ -65,10 +65,11 @@ def _us_per_gemm(m, layers, s, workspace, k, n, qc):
     return sorted(times[4:])[5]
 
 
-def test_time_of_32_rows_on_a_narrow_layer():
+@pytest.mark.parametrize("m,bound", [(16, 1.27), (32, 1.75)])
+def test_time_on_a_narrow_layer(m, bound):
     """Sixteen CTAs per strip, weights larger than L2."""
     k, n, qc = 16384, 1024, 256
     w = synth.make_layer(k, n, qc, 128, seed=1, keep_dequantized=False).to(torch.device("cuda", 0))
     layers = [w.B.clone() for _ in range(32)]
     workspace = torch.zeros(n // 128 * 16, dtype=torch.int32, device="cuda")
-    assert _us_per_gemm(32, layers, w.s, workspace, k, n, qc) <= 1.35 * _us_per_gemm(16, layers, w.s, workspace, k, n, qc)
+    assert _us_per_gemm(m, layers, w.s, workspace, k, n, qc) <= bound * _us_per_gemm(8, layers, w.s, workspace, k, n, qc)

@@ -57,7 +57,7 @@ struct LaunchPlan {
 // `sms` <= 0: the largest grid any device can get (an upper bound for sizing buffers).
 LaunchPlan plan_launches(int M, const Geometry& geo, int sms, int two_launches = -1, bool fewest_tiles = false) {
   LaunchPlan lp;
-  // 129 to 256 rows on a layer with INT4 group scales and up to 48 blocks per CTA: two launches of the kernel for up to 128 rows.
+  // 129 to 256 rows on a layer with INT4 group scales and up to 48 blocks per CTA: two launches of the kernels for up to 128 rows.
   // It multiplies the fp32 sums by the group scales; the other kernel rounds every scaled weight to fp16 first, which costs
   // bits (INT4 columns against 64-bit sums, K = 1024 to 11008: relative error 2.07e-4 here, 2.67e-4 there; with the rounding
   // of the result alone 2.07e-4).  One launch of the other kernel is faster and is the plan of layers without group scales, on
@@ -214,7 +214,7 @@ int mul_impl(const void* A, const void* B, void* C, const void* s, int M, int N,
     p.R = epilogue == kEpilogueResidual ? static_cast<const half*>(residual) + (size_t)m0 * N : nullptr;
     for (int q = 0; q < out.n_out; ++q) p.out.peer[q] = out.peer[q] + (size_t)m0 * out.ld;
     p.M = (M - m0) < rows ? (M - m0) : rows;
-    // The last of several launches may be left with so few rows that the kernel for up to 128 rows is the faster one;
+    // The last of several launches may be left with so few rows that a kernel for up to 128 rows is the faster one;
     // its partials fit (half as many rows, two slots per CTA).
     const bool launch_wide = wide && p.M > kTc5MaxRows;
     const int launch_ctas = wide && !launch_wide ? std::min(ctas, plan_launches(p.M, p.geo, sms).ctas) : ctas;

@@ -131,7 +131,7 @@ FP6M_HD int int4_nibble_pos(int i) { return (i & 1) ? 4 + (i >> 1) : (i >> 1); }
 // Stripe schedule.  Units are ordered strip-major (INT4 strips, then FP6 strips), rows fastest,
 // and weighted by their cost (unit_cost: 8 per INT4 unit, 11 per FP6 unit).  CTA c owns the units
 // [bound[c], bound[c+1]); a strip that is shared by several CTAs is summed in fp32 by one of them:
-// the one in which it ends (kernel for up to 128 rows) or starts (kernel for more).  Replaces the reference's static INT4/FP6 SM split and its stripe
+// the one in which it ends (33 to 128 rows) or starts (fewer and more rows).  Replaces the reference's static INT4/FP6 SM split and its stripe
 // arithmetic (fp6_marlin_cuda_kernel.cu:308-408).
 // ---------------------------------------------------------------------------------------------
 struct Schedule {

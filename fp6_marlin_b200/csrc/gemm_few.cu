@@ -4,13 +4,17 @@
 // memory a CTA allocates 512 columns and passes operands, sums and slots between roles through mbarriers.
 // Here a consumer warp keeps a tile to itself: packed words -> registers -> mma.sync
 // m16n8k16 -> registers, one barrier wait per segment.
-// What bounds it: issue slots.  An m16n8k16 takes 7.4 cycles of an SM quarter's issue, the other instructions about one each
-// (measured), so a segment costs 320 cycles with one tile of eight rows and 450 with two, against 350 that HBM needs
-// for its 8 KB; from 9 rows on the kernel of gemm_team.cu, whose MMAs cost no issue slots, is the faster one.
-// Measured, us per GEMM in a chain of launches, against the tcgen05 kernel that served these sizes before:
-//   4096 x 4096 at 1 row 8.7 -> 6.4, 4096 x 12288 at 5 rows 12.4 -> 9.6, 4096 x 22016 at 5 rows 16.8 -> 14.3, 11008 x 4096 at 5 rows
-//   12.4 -> 9.6, K = N = 8192 at 8 rows 13.8 -> 11.4, 8192 x 57344 at 5 rows 55.0 (16 rows before: 61.9);
-//   with two tiles, at 16 rows: K = N = 8192 13.8 -> 15.3, 8192 x 57344 62 -> 74 (hence the line at 8 rows).
+// What bounds it: an m16n8k16 takes 7.4 cycles of an SM quarter's issue, the other instructions about one each (micro-benchmarks),
+// so the inner loop of a segment needs 320 cycles of issue with one tile of eight rows and 450 with two, against 350 that HBM needs for its
+// 8 KB; from 9 rows on the kernel of gemm_team.cu, whose MMAs cost no issue slots, is the faster one.  In a launch a segment costs 530
+// cycles (from 4096 x 22016 to 8192 x 57344 at 8 rows), so waits between the roles add to that; K = N = 8192 has 43 % of the issue
+// slots busy, and set-up, first data and tail are a third of a CTA's life.
+// Measured, us per GEMM in a chain of launches (256 FP6 columns, group scales, weights larger than L2), against the tcgen05 kernel that served
+// these sizes before, without / with launch overlap:
+//   4096 x 4096 at 1 row 8.7 / 7.7 -> 6.3 / 6.2, 4096 x 12288 at 5 rows 12.85 / 12.35 -> 9.85 / 9.45, 4096 x 22016 at 5 rows 17.9 / 17.6 -> 14.9 /
+//   14.4, 11008 x 4096 at 5 rows 12.8 / 12.85 -> 9.8 / 9.5, K = N = 8192 at 8 rows 14.45 / 14.05 -> 11.75 / 11.4, 8192 x 57344 at 5 rows
+//   66.0 / 65.6 -> 56.4 / 56.2, 16384 x 1024 at 8 rows 12.2 / 10.9 -> 9.1 / 8.9;
+//   with two tiles, at 16 rows with overlap: K = N = 8192 13.8 -> 15.3, 8192 x 57344 62 -> 74 (hence the line at 8 rows).
 //
 // The product is computed transposed, as in the other kernels: W is the 16-row operand (16 weight columns x 16 rows of K), A the
 // 8-column one.  The order of K inside a fragment is free as long as both operands agree, so a thread (g = lane / 4,

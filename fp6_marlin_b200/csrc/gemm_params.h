@@ -54,7 +54,7 @@ struct MulParams {
   int tile_rows;        // kernel for more than 128 rows: rows of a tile
   Schedule sched;
 };
-// Off a 16-byte boundary the 128-row instance of the kernel for up to 128 rows (64 registers a thread) reloads the geometry
+// Off a 16-byte boundary the 128-row instance of the kernel for 33 to 128 rows (64 registers a thread) reloads the geometry
 // piece by piece and spills: 608 instead of 144 bytes of spill loads, K = N = 8192 at 128 rows 29.5 instead of 27.9 us.
 static_assert(offsetof(MulParams, geo) % 16 == 0, "parameter block");
 

@@ -7,16 +7,18 @@
 // tiles, times the group scale in fp32, into registers.  So there are no epilogue warps, no ring of scales, no tiles to zero
 // and no barrier between accumulator and team: program order does it.  One thread issues all MMAs of a tile, hence sums
 // in one order and results that repeat bit for bit.
-// What bounds it: the teams' instructions (expansion 144 per warp and segment, at half rate) and the waits between them; the tensor
-// pipe needs 75 cycles per segment, the issuers 100.  Before the issuers used elect.sync (see elect_one) they needed 1400.
-// Measured, us per GEMM in a chain of launches, against the kernel with epilogue warps that served these sizes before:
-//   at 16 rows, four teams: 4096 x 4096 8.8 -> 8.0, K = N = 8192 13.8 -> 12.6, 8192 x 57344 61.9 -> 51 to 57; at 32 rows K = N = 8192
-//   16.1 -> 15.6;
-//   four teams -> three, on another GPU: 4096 x 4096 8.2 -> 7.5, 4096 x 22016 17.4 -> 15.7, K = N = 8192 13.5 -> 12.4, 8192 x 57344
-//   59.1 -> 54.4, at 32 rows K = N = 8192 15.7 -> 14.6.
+// What bounds it: the teams' instructions (expansion 144 per warp and segment, at half rate) and the waits between them: a segment costs 510
+// cycles (from 4096 x 22016 to 8192 x 57344 at 16 rows), HBM needs 350 for it, the tensor pipe 75, the issuers 100.  Before the issuers used elect.sync (see elect_one) they needed 1400.
+// Measured, us per GEMM in a chain of launches (256 FP6 columns, group scales, weights larger than L2), against the kernel with epilogue warps
+// that served these sizes before, without / with launch overlap:
+//   at 16 rows 4096 x 4096 8.85 / 7.7 -> 7.55 / 6.7, 4096 x 22016 17.9 / 17.7 -> 15.9 / 15.3, 11008 x 4096 12.9 / 12.8 -> 11.4 / 10.7, K = N = 8192
+//   14.6 / 14.15 -> 13.2 / 12.6, 8192 x 57344 66.5 / 66.4 -> 56.7 / 56.4, 16384 x 1024 12.2 / 10.7 -> 10.5 / 9.6;
+//   at 32 rows 4096 x 4096 10.3 / 9.2 -> 9.1 / 8.4, K = N = 8192 16.9 / 16.5 -> 14.85 / 14.5, 8192 x 57344 74.5 -> 61.8, 16384 x 1024 15.9 / 14.8 -> 14.3 / 13.3.
+//   Four teams instead of three, on another GPU: 4096 x 4096 8.2 instead of 7.5, K = N = 8192 13.5 instead of 12.4, 8192 x 57344 59.1 instead of 54.4.
 //
 // A slice (the CTA's blocks of one strip) is finished when a team has expanded its first segment of the next one, so its last
-// MMAs are done by then; the teams pool their sums through shared memory.  Roles: warps 0 and 1 weights (every second segment
+// MMAs are done by then; the teams pool their sums through shared memory, and two of them write the rows out or leave them as a partial.  The
+// CTA's last slice, if its strip goes on in other CTAs, is summed by two or four groups of warps (kSumGroups).  Roles: warps 0 and 1 weights (every second segment
 // each), warp 2 tensor memory, activations and launch epoch, then one MMA issuer per team, then the teams.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

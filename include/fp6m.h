@@ -95,7 +95,7 @@ size_t fp6m_mul_scratch_bytes(int M, int N, int K, int quant_cols, int sms);
 
 /* How fp6m_mul cuts this shape into kernel launches on a device with `sms` multiprocessors (the reference's
  * dispatcher likewise covers M in several launches, fp6_marlin_cuda_kernel.cu:917-948): returns their number;
- * *many_rows_kernel (may be null) = 1 if the kernel for more than 128 rows runs, 0 if the one for up to 128.
+ * *many_rows_kernel (may be null) = 1 if the kernel for more than 128 rows runs, 0 if one of those for up to 128.
  * For group_size = 128; with one scale per column 129 to 256 rows are one launch of the former on every layer. */
 int fp6m_mul_launches(int M, int N, int K, int quant_cols, int sms, int* many_rows_kernel);
 
